@@ -410,6 +410,16 @@ int pcgb_copy_rows_async(void* dst, int64_t dst_pitch, const void* src, int64_t 
  * equal to the hardware conversion). Either output may be NULL. */
 int pcgb_fp64_helpers(const double* x, double* rcp, float* narrowed, int64_t n, void* stream);
 
+/* The damped FP64 solve and the gain-ratio decisions of a float32 fitter, one
+ * system of nparam = 2..6 unknowns per element, exposed for tests: A (H, n)
+ * packed lower triangles, b, s (nparam, n) gradients and steps, f and ftp (n)
+ * costs before and after; x (nparam, n) = the solution for A and b, code =
+ * bits 0-2 step accepted, accepted as very good, predicted reduction < 0 as
+ * the fp32 test decides, bit 3 whether it decides (else FP64 does), bits 4-6
+ * the same from the FP64 test. */
+int pcgb_solve_helpers(int nparam, const float* A, const float* b, const float* s, const float* f, const float* ftp,
+                       double mu, double eta, float* x, int32_t* code, int64_t n, void* stream);
+
 /* Constant initialisation: pars[k][v] = values[k]; a NaN entry means "the
  * voxel's largest sample" (the reference notebooks' S0 start). */
 int pcgb_init_constant(const float* data, int64_t n, int m, int nparam, const double* values, float* pars,

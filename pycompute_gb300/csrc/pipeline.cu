@@ -26,6 +26,31 @@ __global__ void fp64_helpers_kernel(const double* x, double* rcp, float* nar, lo
   if (nar) nar[i] = pcgb::narrow(x[i]);
 }
 
+// The FP64 solve and the gain-ratio decisions of an FP32 fitter, one system per
+// thread: x = the solution, code = bits 0-2 accept, accepted as very good,
+// predicted < 0 as gain_f32 answers, bit 3 whether it does, bits 4-6 the same
+// from gain_f64.
+template <int P>
+__global__ void solve_helpers_kernel(const float* A, const float* b, const float* s, const float* f, const float* ftp,
+                                     float mu, float eta, float* x, int* code, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  constexpr int H = P * (P + 1) / 2;
+  float a[H], g[P], st[P], r[P];
+  for (int k = 0; k < H; ++k) a[k] = A[k * n + i];
+  for (int k = 0; k < P; ++k) {
+    g[k] = b[k * n + i];
+    st[k] = s[k * n + i];
+  }
+  pcgb::gmw81_solve_f32in_f64<P>(a, g, r);
+  for (int k = 0; k < P; ++k) x[k * n + i] = r[k];
+  bool ac, vg, ng, ac2, vg2, ng2;
+  const bool ok = pcgb::gain_f32<P>(f[i], ftp[i], st, g, a, mu, eta, ac, vg, ng);
+  pcgb::gain_f64<P>(f[i], ftp[i], st, g, a, mu, eta, ac2, vg2, ng2);
+  code[i] = int(ac) | int(ac && vg) << 1 | int(ng) << 2 | int(ok) << 3 | int(ac2) << 4 | int(ac2 && vg2) << 5 |
+            int(ng2) << 6;
+}
+
 thread_local std::string g_err;
 int fail(int code, const char* m) {
   g_err = m;
@@ -280,6 +305,27 @@ int pcgb_fp64_helpers(const double* x, double* rcp, float* narrowed, int64_t n, 
   const long long blocks = (n + 255) / 256;
   if (blocks > 0x7fffffffLL) return fail(PCGB_ERANGE, "fp64_helpers: n too large");
   fp64_helpers_kernel<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, rcp, narrowed, n);
+  return cuda_rc();
+}
+
+int pcgb_solve_helpers(int nparam, const float* A, const float* b, const float* s, const float* f, const float* ftp,
+                       double mu, double eta, float* x, int32_t* code, int64_t n, void* stream) {
+  if (nparam < 2 || nparam > 6 || n < 0 || (n > 0 && (!A || !b || !s || !f || !ftp || !x || !code)))
+    return fail(PCGB_EINVAL, "bad solve_helpers arguments");
+  if (n == 0) return PCGB_OK;
+  const long long blocks = (n + 127) / 128;
+  if (blocks > 0x7fffffffLL) return fail(PCGB_ERANGE, "solve_helpers: n too large");
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const auto go = [&](auto kernel) {
+    kernel<<<unsigned(blocks), 128, 0, st>>>(A, b, s, f, ftp, float(mu), float(eta), x, code, n);
+  };
+  switch (nparam) {
+    case 2: go(solve_helpers_kernel<2>); break;
+    case 3: go(solve_helpers_kernel<3>); break;
+    case 4: go(solve_helpers_kernel<4>); break;
+    case 5: go(solve_helpers_kernel<5>); break;
+    default: go(solve_helpers_kernel<6>); break;
+  }
   return cuda_rc();
 }
 

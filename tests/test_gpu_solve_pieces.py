@@ -1,0 +1,150 @@
+"""The FP32 fitter's solve and gain-ratio decisions, piece by piece: the fp32
+gain test decides exactly as FP64 wherever it decides; the solve equals an FP64
+restatement on definite, indefinite, degenerate and badly scaled systems."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from pycompute_gb300 import _lib
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _t(a, dt=None):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+
+
+def _ptr(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def _solve(P, A, b, s, f, ftp, mu=0.25, eta=0.75):
+    n = b.shape[1]
+    args = [_t(v.astype(np.float32)) for v in (A, b, s, f, ftp)]
+    x = torch.empty((P, n), device=DEV)
+    code = torch.empty(n, dtype=torch.int32, device=DEV)
+    _lib.check("pcgb_solve_helpers", _lib.lib().pcgb_solve_helpers(
+        P, *[_ptr(a) for a in args], mu, eta, _ptr(x), _ptr(code), n,
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    return x.cpu().numpy(), code.cpu().numpy()
+
+
+def _gmw64(A, b):
+    """The GMW81 solve (solver.py:23-95, 431-463): fp32 scaling, the rest in double, one system per column."""
+    P, n = b.shape
+    rot = [P - 1] + list(range(P - 1))
+    at = lambda i, j: A[max(i, j) * (max(i, j) + 1) // 2 + min(i, j)]  # noqa: E731
+    with np.errstate(all="ignore"):
+        s = [np.sqrt(np.abs(at(rot[i], rot[i]))) for i in range(P)]
+        L = [[(at(rot[i], rot[j]) / (s[i] * s[j])).astype(np.float64) for j in range(i + 1)] for i in range(P)]
+        y = [(b[rot[i]] / s[i]).astype(np.float64) for i in range(P)]
+        mx = lambda m, v: np.where(v > m, v, m)  # noqa: E731 - a NaN never wins
+        gam, nu = np.zeros(n), np.zeros(n)
+        for i in range(P):
+            gam = mx(gam, np.abs(L[i][i]))
+            for j in range(i):
+                nu = mx(nu, np.abs(L[i][j]))
+        nu = nu / np.sqrt(P * P - 1.0)
+        beta2 = mx(mx(np.full(n, 4e-16), gam), nu)
+        delta = np.where(gam + nu > 1, 4e-16 * (gam + nu), 4e-16)
+        d = []
+        for j in range(P):
+            Lj = [L[j][q] / d[q] for q in range(j)]
+            th = np.zeros(n)
+            for i in range(j + 1, P):
+                for q in range(j):
+                    L[i][j] = L[i][j] - Lj[q] * L[i][q]
+                th = mx(th, np.abs(L[i][j]))
+            L[j][:j] = Lj
+            dj = np.abs(L[j][j])
+            dj = np.where(dj < delta, delta, dj)
+            dj = np.where(dj < th * th / beta2, th * th / beta2, dj)
+            d.append(dj)
+            for i in range(j + 1, P):
+                L[i][i] = L[i][i] - L[i][j] ** 2 / dj
+        for i in range(P):
+            for j in range(i):
+                y[i] = y[i] - L[i][j] * d[j] * y[j]
+            y[i] = y[i] / d[i]
+        for i in reversed(range(P)):
+            for j in range(i + 1, P):
+                y[i] = y[i] - L[j][i] * y[j]
+        x = [None] * P
+        for i in range(P):
+            x[rot[i]] = (y[i] * (np.float32(1) / s[i]).astype(np.float64)).astype(np.float32)
+    return np.stack(x)
+
+
+def _systems(P, n, kind, rng):
+    J = rng.standard_normal((P + 2, P, n))
+    A = np.einsum("kin,kjn->ijn", J, J)
+    for i in range(P):
+        A[i, i] += 0.3
+        if kind == "indefinite":
+            A[i, i] -= rng.uniform(0.0, 2.0 * P, n)
+    scale = {"wide": 30, "huge": 55}.get(kind, 3)
+    e = 2.0 ** rng.integers(-scale, scale + 1, (P, n))
+    A, b = A * e[:, None] * e[None], rng.standard_normal((P, n)) * e
+    if kind == "zeros":
+        for i in range(P):
+            for j in range(i):
+                z = rng.random(n) < 0.5
+                A[i, j][z] = A[j, i][z] = 0.0
+            b[i][rng.random(n) < 0.3] = 0.0
+    A, b = A.astype(np.float32), b.astype(np.float32)
+    if kind == "nan":
+        b[0, ::3] = np.nan
+        A[0, 0, 1::3] = np.inf
+        A[P - 1, 0, 2::3] = A[0, P - 1, 2::3] = np.nan
+    return np.stack([A[i, j] for i in range(P) for j in range(i + 1)]), b
+
+
+@pytest.mark.parametrize("P", [2, 3, 4, 5, 6])
+@pytest.mark.parametrize("kind", ["definite", "indefinite", "wide", "huge", "zeros", "nan"])
+def test_solve_equals_fp64_restatement(P, kind):
+    n = 4099
+    A, b = _systems(P, n, kind, np.random.default_rng(P))
+    z = np.zeros(n)
+    x, _ = _solve(P, A, b, np.zeros((P, n)), z, z)
+    ref = _gmw64(A, b)
+    fine = np.isfinite(ref)
+    np.testing.assert_array_equal(np.isfinite(x), fine)
+    # one float rounding of a solve that is exact to 2^-52 times the pivots' growth (|c| / d <= 1e4 for all but a few
+    # of these random systems); small entries carry the error of the largest scaled one
+    size = np.abs(np.where(fine, ref, 0)) * np.sqrt(np.abs(np.stack([A[i * (i + 1) // 2 + i] for i in range(P)])))
+    with np.errstate(all="ignore"):
+        tol = 2.0 ** -23 * np.abs(ref) + 1e-10 * size.max(0) / np.sqrt(
+            np.abs(np.stack([A[i * (i + 1) // 2 + i] for i in range(P)]))) + 1.5e-45
+        bad = fine & (np.abs(x - ref) > tol)
+    assert bad.mean() < 1e-3, bad.mean()
+
+
+@pytest.mark.parametrize("P", [2, 4, 6])
+@pytest.mark.parametrize("mu,eta", [(0.25, 0.75), (0.0, 0.75), (-0.5, 2.0)])
+def test_fp32_gain_decides_as_fp64(P, mu, eta):
+    rng = np.random.default_rng(17 + P)
+    n = 1 << 18
+    A, b = _systems(P, n, "definite", rng)
+    s = rng.standard_normal((P, n)) * 2.0 ** rng.integers(-24, 3, n) / np.sqrt(
+        np.stack([A[i * (i + 1) // 2 + i] for i in range(P)]))
+    s32 = s.astype(np.float32).astype(np.float64)
+    pred = np.zeros(n)
+    for i in range(P):
+        pred += s32[i] * b[i]
+        for j in range(i + 1):
+            pred -= A[i * (i + 1) // 2 + j].astype(np.float64) * s32[i] * s32[j] * (0.5 if i == j else 1.0)
+    # actual reductions around both thresholds (some exactly on the rounded threshold), ties, noise and non-finite costs
+    f = rng.uniform(0.0, 1.0, n) * np.abs(pred) * 8
+    k = rng.integers(0, 8, n)
+    ftp = f - np.select([k == 0, k == 1, k == 2, k == 3], [2 * mu * pred * (1 + rng.normal(0, 1e-6, n)),
+                                                             2 * eta * pred * (1 + rng.normal(0, 1e-6, n)),
+                                                             np.zeros(n), 2 * eta * pred], rng.normal(0, 2, n) * pred)
+    ftp[::97], f[1::97], s[:, 2::97] = np.nan, np.inf, 0.0
+    _, code = _solve(P, A, b, s, f, ftp, mu, eta)
+    told = (code & 8) != 0
+    np.testing.assert_array_equal((code & 7)[told], (code >> 4)[told])
+    regular = (np.arange(n) % 97 > 2) & (k > 3)
+    assert told[regular].mean() > 0.97
