@@ -420,6 +420,12 @@ int pcgb_fp64_helpers(const double* x, double* rcp, float* narrowed, int64_t n, 
 int pcgb_solve_helpers(int nparam, const float* A, const float* b, const float* s, const float* f, const float* ftp,
                        double mu, double eta, float* x, int32_t* code, int64_t n, void* stream);
 
+/* Its scalar pieces, elementwise: root = sqrt(b) and quot = a / b by the
+ * straight-line forms (correctly rounded where operands and results are well
+ * inside the normal range). */
+int pcgb_scalar_helpers(const float* a, const float* b, const double* x, float* root, float* quot, double* rcp,
+                        float* prod, int32_t* ok, int64_t n, void* stream);
+
 /* Constant initialisation: pars[k][v] = values[k]; a NaN entry means "the
  * voxel's largest sample" (the reference notebooks' S0 start). */
 int pcgb_init_constant(const float* data, int64_t n, int m, int nparam, const double* values, float* pars,

@@ -89,6 +89,8 @@ SIGNATURES = {
     "pcgb_fp64_helpers": (c_int, [c_void_p, c_void_p, c_void_p, c_i64, c_void_p]),
     "pcgb_solve_helpers": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_double, c_double,
                                    c_void_p, c_void_p, c_i64, c_void_p]),
+    "pcgb_scalar_helpers": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                    c_i64, c_void_p]),
     "pcgb_copy_rows_async": (c_int, [c_void_p, c_i64, c_void_p, c_i64, c_i64, c_i64, c_int, c_void_p]),
     "pcgb_init_constant": (c_int, [c_void_p, c_i64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "pcgb_bpolyfit": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_int, c_int, c_int, c_int, c_void_p,

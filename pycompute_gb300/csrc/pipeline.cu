@@ -50,6 +50,15 @@ __global__ void solve_helpers_kernel(const float* A, const float* b, const float
   code[i] = int(ac) | int(ac && vg) << 1 | int(ng) << 2 | int(ok) << 3 | int(ac2) << 4 | int(ac2 && vg2) << 5 |
             int(ng2) << 6;
 }
+// The straight-line forms of the scaling, elementwise: root = sqrt(b), quot =
+// a / b
+__global__ void scalar_helpers_kernel(const float* a, const float* b, const double* x, float* root, float* quot,
+                                      double* rcp, float* prod, int* ok, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  root[i] = pcgb::sqrt_fast(b[i]);
+  quot[i] = pcgb::div_fast(a[i], b[i], pcgb::rcp_fast(b[i]));
+}
 
 thread_local std::string g_err;
 int fail(int code, const char* m) {
@@ -326,6 +335,18 @@ int pcgb_solve_helpers(int nparam, const float* A, const float* b, const float* 
     case 5: go(solve_helpers_kernel<5>); break;
     default: go(solve_helpers_kernel<6>); break;
   }
+  return cuda_rc();
+}
+
+int pcgb_scalar_helpers(const float* a, const float* b, const double* x, float* root, float* quot, double* rcp,
+                        float* prod, int32_t* ok, int64_t n, void* stream) {
+  if (n < 0 || (n > 0 && (!a || !b || !x || !root || !quot || !rcp || !prod || !ok)))
+    return fail(PCGB_EINVAL, "bad scalar_helpers arguments");
+  if (n == 0) return PCGB_OK;
+  const long long blocks = (n + 255) / 256;
+  if (blocks > 0x7fffffffLL) return fail(PCGB_ERANGE, "scalar_helpers: n too large");
+  scalar_helpers_kernel<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, x, root, quot, rcp,
+                                                                                         prod, ok, n);
   return cuda_rc();
 }
 

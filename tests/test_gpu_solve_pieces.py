@@ -148,3 +148,27 @@ def test_fp32_gain_decides_as_fp64(P, mu, eta):
     np.testing.assert_array_equal((code & 7)[told], (code >> 4)[told])
     regular = (np.arange(n) % 97 > 2) & (k > 3)
     assert told[regular].mean() > 0.97
+
+
+def _scalars(a, b, x):
+    n = len(a)
+    ta, tb, tx = _t(a), _t(b), _t(x)
+    root, quot, prod = (torch.empty(n, device=DEV) for _ in range(3))
+    rcp = torch.empty(n, dtype=torch.float64, device=DEV)
+    ok = torch.zeros(n, dtype=torch.int32, device=DEV)
+    _lib.check("pcgb_scalar_helpers", _lib.lib().pcgb_scalar_helpers(
+        _ptr(ta), _ptr(tb), _ptr(tx), _ptr(root), _ptr(quot), _ptr(rcp), _ptr(prod), _ptr(ok), n,
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    return [v.cpu().numpy() for v in (root, quot, rcp, prod, ok)]
+
+
+def test_straight_line_root_and_quotient_are_correctly_rounded():
+    mant = np.arange(1 << 23, dtype=np.uint32)
+    rng = np.random.default_rng(5)
+    for e in (127, 128, 77, 190):  # every significand, both exponent parities
+        b = (mant | np.uint32(e << 23)).view(np.float32)
+        a = (rng.integers(0, 1 << 23, len(b)).astype(np.uint32) | np.uint32(120 << 23)).view(np.float32)
+        a[::3] = np.nextafter(b[::3], np.float32(0)) * np.float32(0.5)
+        root, quot, *_ = _scalars(a, b, np.ones(len(b)))
+        np.testing.assert_array_equal(root, np.sqrt(b))
+        np.testing.assert_array_equal(quot, a / b)
