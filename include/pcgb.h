@@ -422,7 +422,9 @@ int pcgb_solve_helpers(int nparam, const float* A, const float* b, const float* 
 
 /* Its scalar pieces, elementwise: root = sqrt(b) and quot = a / b by the
  * straight-line forms (correctly rounded where operands and results are well
- * inside the normal range). */
+ * inside the normal range);
+ * rcp = 1/x as pcgb_fp64_helpers computes it, in integer arithmetic, where ok
+ * bit 0 is set; prod = float(x * a) rounded twice, where ok bit 1 is set. */
 int pcgb_scalar_helpers(const float* a, const float* b, const double* x, float* root, float* quot, double* rcp,
                         float* prod, int32_t* ok, int64_t n, void* stream);
 

@@ -58,6 +58,7 @@ __global__ void scalar_helpers_kernel(const float* a, const float* b, const doub
   if (i >= n) return;
   root[i] = pcgb::sqrt_fast(b[i]);
   quot[i] = pcgb::div_fast(a[i], b[i], pcgb::rcp_fast(b[i]));
+  ok[i] = int(pcgb::rcp64_int(x[i], rcp[i])) | int(pcgb::scale_narrow(x[i], a[i], prod[i])) << 1;
 }
 
 thread_local std::string g_err;

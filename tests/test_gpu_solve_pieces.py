@@ -172,3 +172,32 @@ def test_straight_line_root_and_quotient_are_correctly_rounded():
         root, quot, *_ = _scalars(a, b, np.ones(len(b)))
         np.testing.assert_array_equal(root, np.sqrt(b))
         np.testing.assert_array_equal(quot, a / b)
+
+
+def test_integer_reciprocal_and_fp32_product_equal_the_fp64_ones():
+    rng = np.random.default_rng(6)
+    n = 1 << 22
+    m = rng.uniform(1.0, 2.0, n)
+    m[::5] = 1.0 + rng.integers(0, 1 << 12, len(m[::5])) * 2.0 ** -52   # a seed that starts at a power of two
+    m[1::5] = 2.0 - rng.integers(1, 1 << 12, len(m[1::5])) * 2.0 ** -52
+    m[2::5] = m[2::5].astype(np.float32)
+    x = np.ldexp(m, rng.integers(-130, 130, n))
+    a = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-40, 40, n)).astype(np.float32)
+    x = np.where(np.arange(n) % 11 == 0, -x, x)
+    x[:8] = [0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 1e300, 1e-300]
+    _, _, rcp, prod, ok = _scalars(a, np.ones(n, np.float32), x)
+    want = torch.empty(n, dtype=torch.float64, device=DEV)
+    tx = _t(x)
+    _lib.check("pcgb_fp64_helpers", _lib.lib().pcgb_fp64_helpers(_ptr(tx), _ptr(want), None, n, ctypes.c_void_p(
+        torch.cuda.current_stream().cuda_stream)))
+    told = (ok & 1) != 0
+    np.testing.assert_array_equal(rcp.view(np.int64)[told], want.cpu().numpy().view(np.int64)[told])
+    assert not told[:8].any() and not told[x < 0].any()
+    mid = (np.abs(np.log2(np.abs(np.where(x == 0, 1, x)))) < 100) & (x > 0)
+    assert told[mid].mean() > 0.99
+    with np.errstate(all="ignore"):
+        both = (x * a.astype(np.float64)).astype(np.float32)
+    told = (ok & 2) != 0
+    np.testing.assert_array_equal(prod.view(np.int32)[told], both.view(np.int32)[told])
+    near = np.abs(np.log2(np.abs(np.where(x == 0, 1, x)))) < 25
+    assert told[near & np.isfinite(x) & (x != 0)].mean() > 0.99 and not told[:8].any()
