@@ -126,7 +126,7 @@ bool is_lm_slot(int slot) {
          slot == K_LMW_C1_B1;
 }
 
-constexpr int kLmMinBlocks = 6;
+constexpr int kLmMinBlocks = 7;
 // the warm LM with the check as its epilogue (group 4): two iterations and an
 // epilogue per voxel gain from one more block (IVIM-16, 16.7 M voxels, whole
 // warm step: 6 blocks 8.40 ms, 7 blocks 8.30 ms, 8 blocks 8.35 ms)
