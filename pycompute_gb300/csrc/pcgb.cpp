@@ -59,7 +59,7 @@ enum KernelSlot {
   K_SEARCH_C1, K_SEARCH_C0, K_RS_C1_B1, K_RS_C1_B0, K_RS_C0_B1, K_RS_C0_B0,
   K_LMQ_C1_B1, K_LMQ_C1_B0, K_LMQ_C0_B1, K_LMQ_C0_B0, K_CHECK_C1, K_CHECK_C0, K_SELECT_C1, K_SELECT_C0,
   K_LMC_C1_B1, K_LMC_C1_B0, K_LMC_C0_B1, K_LMC_C0_B0, K_LMS_C1_B1, K_LMS_C1_B0, K_LMS_C0_B1, K_LMS_C0_B0,
-  K_LMW_C1_B1, K_LMW_C1_B0, K_LMW_C0_B1, K_LMW_C0_B0, K_COUNT
+  K_LMW_C1_B1, K_LMW_C1_B0, K_LMW_C0_B1, K_LMW_C0_B0, K_LMF, K_COUNT
 };
 const char* kKernelNames[K_COUNT] = {"pcgb_lm_c1_b1", "pcgb_lm_c1_b0", "pcgb_lm_c0_b1", "pcgb_lm_c0_b0",
                                      "pcgb_cost_c1",  "pcgb_cost_c0",  "pcgb_gmw81",    "pcgb_eval_c1",
@@ -69,7 +69,7 @@ const char* kKernelNames[K_COUNT] = {"pcgb_lm_c1_b1", "pcgb_lm_c1_b0", "pcgb_lm_
                                      "pcgb_check_c0", "pcgb_select_c1", "pcgb_select_c0", "pcgb_lmc_c1_b1",
                                      "pcgb_lmc_c1_b0", "pcgb_lmc_c0_b1", "pcgb_lmc_c0_b0", "pcgb_lms_c1_b1",
                                      "pcgb_lms_c1_b0", "pcgb_lms_c0_b1", "pcgb_lms_c0_b0", "pcgb_lmw_c1_b1",
-                                     "pcgb_lmw_c1_b0", "pcgb_lmw_c0_b1", "pcgb_lmw_c0_b0"};
+                                     "pcgb_lmw_c1_b0", "pcgb_lmw_c0_b1", "pcgb_lmw_c0_b0", "pcgb_lmf"};
 
 constexpr int kDefaultBlock = 128;
 constexpr int kMaxBlock = 256;
@@ -81,8 +81,8 @@ constexpr int64_t kMaxMultiChunks = int64_t(1) << 31;
 struct pcgb_fitter {
   int P = 0, C = 0, M = 0, dtype = 0, sdtype = 0;
   int device = -1;
-  cudaLibrary_t lib[5] = {};  // one per kernel group, loaded on first use
-  int lm_min_blocks[5] = {};  // occupancy hint the group's LM kernels were built with (0: none)
+  cudaLibrary_t lib[6] = {};  // one per kernel group, loaded on first use
+  int lm_min_blocks[6] = {};  // occupancy hint the group's LM kernels were built with (0: none)
   cudaKernel_t k[K_COUNT] = {};
   std::string source, structname, cache_dir;
   std::mutex mu;
@@ -96,12 +96,14 @@ namespace {
 // solve), 1 the searches, 2 the refill schedule and the warm-start fallback
 // check (also as the LM's epilogue), 3 the fallback refit with the select as
 // its epilogue, 4 the warm LM from a fresh start with the check as its
-// epilogue. A group's LM kernels share one register cap (dropped when one of
+// epilogue, 5 the flow schedule of long fits of many voxels. A group's LM kernels share one register cap (dropped when one of
 // them would spill too much), so the refit and the fresh warm LM sit apart
 // from the kernels whose larger state cannot take the cap.
-constexpr int kGroups = 5;
+constexpr int kGroups = 6;
 int group_of(int slot) {
   switch (slot) {
+    case K_LMF:
+      return 5;
     case K_LMW_C1_B1: case K_LMW_C1_B0: case K_LMW_C0_B1: case K_LMW_C0_B0:
       return 4;
     case K_SEARCH_C1: case K_SEARCH_C0: case K_RS_C1_B1: case K_RS_C1_B0: case K_RS_C0_B1: case K_RS_C0_B0:
@@ -118,32 +120,52 @@ int group_of(int slot) {
 
 // The LM kernels for a shared protocol and shared bounds (the common case,
 // the variant with the fewest registers) are first built for at least
-// kLmMinBlocks resident 128-thread blocks per SM (a register cap: more warps
-// to hide the FP64 pipe's latency); a model whose capped kernels would spill
+// kLmMinBlocks times 128 resident threads per SM (a register cap: more warps to
+// hide latency; IVIM-10, 1 M voxels x 20 iterations, 4 to 8 times 1784, 1648,
+// 1602, 1560, 1542 us, but 8 spills more than kLmMaxSpillBytes); a model whose capped kernels would spill
 // more than kLmMaxSpillBytes per thread is rebuilt without the cap.
 bool is_lm_slot(int slot) {
   return slot == K_LM_C1_B1 || slot == K_LMQ_C1_B1 || slot == K_LMC_C1_B1 || slot == K_LMS_C1_B1 ||
-         slot == K_LMW_C1_B1;
+         slot == K_LMW_C1_B1 || slot == K_LMF;
 }
 
+// kernels that run LM iterations, one voxel per thread
+bool is_fit_slot(int slot) {
+  return (slot >= K_LM_C1_B1 && slot <= K_LM_C0_B0) || (slot >= K_LMC_C1_B1 && slot <= K_LMF);
+}
+
+// their threads per block unless the caller says: single warps spread evenly over
+// the SMs and leave them one by one (65,536 IVIM-10 voxels x 10 iterations, all
+// FP64: 128, 64, 32 threads 2607, 2349, 2349 us; 50,000 x 50: 346, 342, 337)
+constexpr int kFitBlock = 32;
 constexpr int kLmMinBlocks = 7;
-// the warm LM with the check as its epilogue (group 4): two iterations and an
-// epilogue per voxel gain from one more block (IVIM-16, 16.7 M voxels, whole
-// warm step: 6 blocks 8.40 ms, 7 blocks 8.30 ms, 8 blocks 8.35 ms)
+// the warm LM with the check as its epilogue (group 4; IVIM-16, 16.7 M voxels: 6,
+// 7, 8 times 4.27, 4.05, 4.52 ms)
 constexpr int kLmWarmMinBlocks = 7;
-// the refit of the flagged voxels with the select as its epilogue (group 3):
-// 6, 7 and 8 blocks measured within 0.3 % on the whole warm step (8.32, 8.32,
-// 8.34 ms)
+// the refit of the flagged voxels with the select as its epilogue (group 3; 43 k
+// voxels x 8 iterations: 6, 8 times 96, 93 us, but 8 spills more than
+// kLmMaxSpillBytes)
 constexpr int kLmRefitMinBlocks = 6;
+// the flow schedule (4 M IVIM-10 voxels x 100 iterations: 5, 6, 7, 8 times 17.5,
+// 17.2, 17.5, 18.1 ms)
+constexpr int kLmFlowMinBlocks = 6;
+// A fit runs the flow schedule (lm_flow_grid) from 64 iterations on and where a
+// resident thread has 128 voxel-iterations beyond the 40th, about where the
+// first voxels come to rest: a pass there costs 20 to 35 % more than a grid
+// iteration (larger code, warps out of step) until voxels finish. us, grid and
+// flow: IVIM-10 x 100, 0.15 M voxels 1364, 1451, 0.3 M 2317, 2105, 1.2 M 8388,
+// 6090; x 64, 0.6 M 2784, 2820, 1.2 M 5417, 5129; x 50, 1.2 M 4264, 4731;
+// IVIM-21 x 64, 4.8 M 29966, 28126; T2*-16 x 64, 0.6 M 2572, 1311.
+constexpr int kFlowMinIters = 64;
+constexpr int kFlowRestIters = 40;
+constexpr double kFlowMinWork = 128.0;
 constexpr int lm_min_blocks_of(int g) {
-  return g == 1 ? 0 : (g == 4 ? kLmWarmMinBlocks : (g == 3 ? kLmRefitMinBlocks : kLmMinBlocks));
+  return g == 1 ? 0 : (g == 4 ? kLmWarmMinBlocks : (g == 3 ? kLmRefitMinBlocks : (g == 5 ? kLmFlowMinBlocks : kLmMinBlocks)));
 }
 constexpr int kLmMaxThreads = 128;
-// Spilled words stay in L1 and cost less than the occupancy gain up to a few
-// hundred bytes per thread (measured with the sample loops rolled, 8.4 M
-// voxels: 5 -> 6 blocks per SM, 0 -> 84 bytes of spills, IVIM-16 x 8
-// iterations 11.86 -> 11.68 ms, IVIM-10 x 20 flat; 7 and 8 blocks within 1 %);
-// past this the cap is dropped.
+// Spilled words (and the samples that the loops index) stay in L1 and cost less
+// than the occupancy gains up to a few hundred bytes per thread; past this the
+// cap is dropped.
 constexpr size_t kLmMaxSpillBytes = 256;
 
 std::string program_source(const char* model_source, const char* model_struct, int P, int C, int M, int dtype,
@@ -161,6 +183,9 @@ std::string program_source(const char* model_source, const char* model_struct, i
                                                   std::to_string(lm_min_blocks) + ")"
                                             : std::string(bounds);
   const bool g0 = group == 0, g1 = group == 1, g2 = group == 2, g3 = group == 3, g4 = group == 4;
+  if (group == 5 && dtype == PCGB_DTYPE_F32 && sdtype == PCGB_DTYPE_F64)
+    s << "extern \"C\" __global__ void " << lmb << " pcgb_lmf(const PcgbLmParams a) { pcgb::lm_flow_grid<PcgbModel, " << M
+      << ", float, double>(a); }\n";
   for (int c = 1; c >= 0 && g0; --c)
     for (int b = 1; b >= 0; --b)
       s << "extern \"C\" __global__ void " << (c && b ? lmb : std::string(bounds)) << " pcgb_lm_c" << c << "_b" << b
@@ -321,6 +346,18 @@ int launch(pcgb_fitter* ft, KernelSlot slot, PcgbLmParams prm, int64_t n, int bl
   return PCGB_OK;
 }
 
+// Blocks of `block` threads of a kernel that are resident on the current device at once.
+int64_t resident_blocks(cudaKernel_t kern, int block) {
+  int per_sm = 0, dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(kern), block, 0) !=
+          cudaSuccess ||
+      per_sm < 1)
+    per_sm = 1;
+  return int64_t(per_sm) * (sms > 0 ? sms : 1);
+}
+
 // launch() for work whose item count lives on the device (prm.n_items_dev,
 // at most n): the kernel strides over its items, so the grid holds only as
 // many blocks as are resident at once instead of one block per possible item
@@ -331,15 +368,11 @@ int launch_resident(pcgb_fitter* ft, KernelSlot slot, PcgbLmParams prm, int64_t 
   block = lm_block(ft, slot, block);
   if (block > kMaxBlock || block % 32) return fail(PCGB_EINVAL, "block must be a multiple of 32 up to %d", kMaxBlock);
   if (n == 0) return PCGB_OK;
-  int per_sm = 0, dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(kern), block, 0);
-  if (e != cudaSuccess || per_sm < 1) per_sm = 1;
   int grid = grid_for(n, block);
-  if (int64_t(per_sm) * (sms > 0 ? sms : 1) < grid) grid = per_sm * (sms > 0 ? sms : 1);
+  const int64_t resident = resident_blocks(kern, block);
+  if (resident < grid) grid = int(resident);
   void* args[] = {&prm};
-  e = cudaLaunchKernel(reinterpret_cast<const void*>(kern), dim3(grid), dim3(block), args, 0,
+  const cudaError_t e = cudaLaunchKernel(reinterpret_cast<const void*>(kern), dim3(grid), dim3(block), args, 0,
                        static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, kKernelNames[slot]);
   return PCGB_OK;
@@ -480,7 +513,7 @@ size_t max_lm_spill_bytes(const std::string& log) {
 // Threads per block for an LM launch: kernels built with the occupancy hint
 // take at most kLmMaxThreads (the per-voxel results do not depend on it).
 int lm_block(const pcgb_fitter* ft, int slot, int block) {
-  if (block <= 0) block = kDefaultBlock;
+  if (block <= 0) block = is_fit_slot(slot) ? kFitBlock : kDefaultBlock;
   if (is_lm_slot(slot) && ft->lm_min_blocks[group_of(slot)] > 0 && block > kLmMaxThreads) block = kLmMaxThreads;
   return block;
 }
@@ -556,6 +589,7 @@ int pcgb_fitter_compile(const char* model_source, const char* model_struct, int 
   if (int rc = validate_create(model_source, model_struct, nparam, nconst, ndata, dtype, solve_dtype)) return rc;
   std::string all;
   for (int g = 0; g < kGroups; ++g) {
+    if (g == 5 && (dtype != PCGB_DTYPE_F32 || solve_dtype != PCGB_DTYPE_F64)) continue;  // no kernel in it
     std::vector<char> cubin;
     std::string log;
     if (int rc = get_cubin(model_source, model_struct, nparam, nconst, ndata, dtype, solve_dtype, cache_dir, g,
@@ -791,6 +825,23 @@ struct FallbackArgs {
   int8_t* which = nullptr;
 };
 
+// Whether a whole-volume fit runs the flow schedule (see kFlowMinIters), which
+// only pays where its kernel keeps the register cap. A kernel that is not loaded
+// yet is not loaded under stream capture.
+static bool flow_pays(pcgb_fitter* ft, int64_t n, int iters, void* stream) {
+  if (ft->dtype != PCGB_DTYPE_F32 || ft->sdtype != PCGB_DTYPE_F64 || iters < kFlowMinIters) return false;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const double threads = double(kLmMaxThreads) * kLmFlowMinBlocks * (sms > 0 ? sms : 1);
+  if (double(n) * (iters - kFlowRestIters) < kFlowMinWork * threads) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap) != cudaSuccess) return false;
+  if (cap != cudaStreamCaptureStatusNone && !ft->k[K_LMF]) return false;
+  cudaKernel_t kern = nullptr;
+  return kernel_of(ft, K_LMF, &kern) == PCGB_OK && ft->lm_min_blocks[5] > 0;
+}
+
 static int lm_run_impl(pcgb_fitter* ft, const void* consts, int64_t consts_stride, const void* data,
                        const void* lower_bound, const void* upper_bound, int64_t bounds_stride, double tol, double mu,
                        double eta, double acc, double dec, void* params, void* step, void* lam, int8_t* step_type,
@@ -912,6 +963,8 @@ static int lm_run_impl(pcgb_fitter* ft, const void* consts, int64_t consts_strid
     if (n_items_dev) return launch_resident(ft, slot, prm, n_items, block, stream);
     return launch(ft, slot, prm, n_items, block, stream);
   }
+  if (block <= 0 && slot == K_LM_C1_B1 && !flags && flow_pays(ft, nprobs, iters, stream))
+    return launch_resident(ft, K_LMF, prm, nprobs, block, stream);
   return launch(ft, slot, prm, nprobs, block, stream);
 }
 

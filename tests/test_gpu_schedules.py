@@ -1,0 +1,43 @@
+"""The launch schedules agree bit for bit: the flow schedule of long fits of many
+voxels with the grid schedule, which runs every iteration."""
+import pytest
+import torch
+
+from pycompute_gb300 import Expr, SecondOrderLevenbergMarquardt, pipeline, synth
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _state(s):
+    return {k: getattr(s, k) for k in ("pars_t", "first_f", "last_f", "f_t", "lam_t", "step_type_t", "step_t", "iters_t")}
+
+
+def _same(a, b):
+    for k in a:
+        x, y = a[k], b[k]
+        x, y = (v.view(torch.int32) if v.dtype == torch.float32 else v for v in (x, y))
+        assert torch.equal(x, y), (k, int((x != y).sum()))
+
+
+@pytest.mark.parametrize("workload,iters,kw", [
+    (synth.ivim, 100, {}), (synth.ivim, 130, dict(dec=1.0)), (synth.ivim, 120, dict(dec=3.7, acc=0.5)),
+    (synth.ivim, 110, dict(dec=0.7)), (synth.t2star, 100, dict(tol=1e-30)), (synth.vfa_t1, 150, {}),
+    (synth.ivim, 260, dict(mu=0.0, eta=0.1)), (synth.biexp_t2, 100, {})])
+def test_flow_equals_grid(workload, iters, kw):
+    w = workload()
+    n = 262147  # 128 voxel-iterations past the 40th per resident thread, ragged
+    _, data = pipeline.synth_gpu(w, n, seed=3, device=DEV)
+    data[:, 5::1001] = float("nan")
+    data[:, 6::1003] = 0.0
+    got = []
+    for block in (0, 128):  # a block size asks for the grid schedule
+        s = SecondOrderLevenbergMarquardt(Expr(w.expr, w.pars, w.consts), None, w.M, torch.float32)
+        s.setup(pipeline.init_constant(data, w.init_values), list(w.protocol), data, list(w.lb), list(w.ub))
+        s.step_type_t[0, ::17] = 0   # converged before the call
+        s.step_type_t[0, 1::17] = 4  # left by an earlier run after a rejected step
+        s.lam_t[0, 2::19] = 1e20     # a damping from which every step is too small
+        s.run(iters, block=block, **kw)
+        torch.cuda.synchronize()
+        got.append(_state(s))
+    _same(*got)
