@@ -6,6 +6,7 @@
 #define PCGB_MAX_PARAMS 8
 #define PCGB_MAX_PROTOCOL 256
 #define PCGB_MAX_MODELS 8
+#define PCGB_MAX_SEARCH_BLOCK 128  // threads per block of the random search
 
 // PcgbLmParams.flags of an LM run
 #define PCGB_LM_FRESH 1      // every voxel starts at lam = lam_start, step_type = 1; lam, f, step are not read
@@ -29,6 +30,7 @@ struct PcgbLmParams {
   void* best_p;            // (P, N) best point of a search, in/out
   void* best_f;            // (N) its cost, in/out
   unsigned long long seed; // random-search draws: counter-based stream per (seed, voxel, draw)
+  int draw_threads;        // threads that share a voxel's draws (1..blockDim.x)
   int lm_iters;            // LM iterations per draw (0: plain random search)
   int* iters_done;         // (N) in/out iteration counter or null
   unsigned int* work;      // voxel work counter of the persistent schedule (zeroed by the host) or null

@@ -126,7 +126,7 @@ int group_of(int slot) {
 // more than kLmMaxSpillBytes per thread is rebuilt without the cap.
 bool is_lm_slot(int slot) {
   return slot == K_LM_C1_B1 || slot == K_LMQ_C1_B1 || slot == K_LMC_C1_B1 || slot == K_LMS_C1_B1 ||
-         slot == K_LMW_C1_B1 || slot == K_LMF;
+         slot == K_LMW_C1_B1 || slot == K_LMF || slot == K_RS_C1_B1;
 }
 
 // kernels that run LM iterations, one voxel per thread
@@ -146,6 +146,9 @@ constexpr int kLmWarmMinBlocks = 7;
 // voxels x 8 iterations: 6, 8 times 96, 93 us, but 8 spills more than
 // kLmMaxSpillBytes)
 constexpr int kLmRefitMinBlocks = 6;
+// the random search (16,001 IVIM-21 voxels x 10 draws x 20 iterations: 4, 5 times
+// 964, 739 us; 6 spills more than kLmMaxSpillBytes)
+constexpr int kLmSearchMinBlocks = 5;
 // the flow schedule (4 M IVIM-10 voxels x 100 iterations: 5, 6, 7, 8 times 17.5,
 // 17.2, 17.5, 18.1 ms)
 constexpr int kLmFlowMinBlocks = 6;
@@ -160,7 +163,7 @@ constexpr int kFlowMinIters = 64;
 constexpr int kFlowRestIters = 40;
 constexpr double kFlowMinWork = 128.0;
 constexpr int lm_min_blocks_of(int g) {
-  return g == 1 ? 0 : (g == 4 ? kLmWarmMinBlocks : (g == 3 ? kLmRefitMinBlocks : (g == 5 ? kLmFlowMinBlocks : kLmMinBlocks)));
+  return g == 1 ? kLmSearchMinBlocks : (g == 4 ? kLmWarmMinBlocks : (g == 3 ? kLmRefitMinBlocks : (g == 5 ? kLmFlowMinBlocks : kLmMinBlocks)));
 }
 constexpr int kLmMaxThreads = 128;
 // Spilled words (and the samples that the loops index) stay in L1 and cost less
@@ -224,7 +227,7 @@ std::string program_source(const char* model_source, const char* model_struct, i
       << (c ? "true" : "false") << ">(a); }\n";
   for (int c = 1; c >= 0 && g1; --c)
     for (int b = 1; b >= 0; --b)
-      s << "extern \"C\" __global__ void " << bounds << " pcgb_rs_c" << c << "_b" << b
+      s << "extern \"C\" __global__ void " << (c && b ? lmb : std::string("__launch_bounds__(128)")) << " pcgb_rs_c" << c << "_b" << b
         << "(const PcgbLmParams a) { pcgb::random_search_grid<PcgbModel, " << M << ", " << ta << ", " << ts << ", "
         << (c ? "true" : "false") << ", " << (b ? "true" : "false") << ">(a); }\n";
   for (int c = 1; c >= 0 && g2; --c) {
@@ -376,6 +379,35 @@ int launch_resident(pcgb_fitter* ft, KernelSlot slot, PcgbLmParams prm, int64_t 
                        static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, kKernelNames[slot]);
   return PCGB_OK;
+}
+
+// Random search: the draws of a voxel over as many threads as make the fewest
+// rounds of draws times waves of resident blocks (fewer threads where equal: the
+// signals are then read less often).
+int launch_search(pcgb_fitter* ft, KernelSlot slot, PcgbLmParams prm, void* stream) {
+  cudaKernel_t kern = nullptr;
+  if (int rc = kernel_of(ft, slot, &kern)) return rc;
+  const int64_t n = prm.N;
+  if (n == 0) return PCGB_OK;
+  constexpr int block = PCGB_MAX_SEARCH_BLOCK;
+  const int64_t resident = resident_blocks(kern, block);
+  const auto blocks = [&](int d) { return (n + block / d - 1) / (block / d); };
+  double least = -1.0;
+  for (int d = 1; d <= block && d <= (prm.iters > 1 ? prm.iters : 1); ++d) {
+    const double waves = double(blocks(d)) / double(resident);
+    const double cost = double((prm.iters + d - 1) / d) * (waves > 1.0 ? waves : 1.0);
+    if (least < 0.0 || cost < 0.98 * least) {
+      least = cost;
+      prm.draw_threads = d;
+    }
+  }
+  const int64_t grid = blocks(prm.draw_threads);
+  if (grid > 0x7fffffff) return fail(PCGB_ERANGE, "too many voxels for one search launch");
+  prm.n_items = n;
+  void* args[] = {&prm};
+  const cudaError_t e = cudaLaunchKernel(reinterpret_cast<const void*>(kern), dim3(unsigned(grid)), dim3(block), args,
+                                         0, static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? PCGB_OK : cuda_fail(e, kKernelNames[slot]);
 }
 
 int fill_protocol(const pcgb_fitter* ft, PcgbLmParams& prm, int64_t cstride, int64_t n, const double* protocol,
@@ -597,7 +629,7 @@ int pcgb_fitter_compile(const char* model_source, const char* model_struct, int 
       return rc;
     // the register-capped LM kernels spill too much for this model: the
     // runtime will load the uncapped build, so compile (and cache) it too
-    if (g != 1 && max_lm_spill_bytes(log) > kLmMaxSpillBytes) {
+    if (max_lm_spill_bytes(log) > kLmMaxSpillBytes) {
       all += log;
       log.clear();
       if (int rc = get_cubin(model_source, model_struct, nparam, nconst, ndata, dtype, solve_dtype, cache_dir, g, 0,
@@ -1321,7 +1353,7 @@ int pcgb_random_search(pcgb_fitter* ft, const void* consts, int64_t consts_strid
   set_lm_constants(prm, tol, mu, eta, acc, dec);
   const KernelSlot slot = consts_stride == 0 ? (bounds_stride == 0 ? K_RS_C1_B1 : K_RS_C1_B0)
                                              : (bounds_stride == 0 ? K_RS_C0_B1 : K_RS_C0_B0);
-  return launch(ft, slot, prm, nprobs, 0, stream);
+  return launch_search(ft, slot, prm, stream);
 }
 
 int pcgb_gmw81_solve(pcgb_fitter* ft, const void* mat, const void* rhs, void* sol, int64_t nprobs, void* stream) {

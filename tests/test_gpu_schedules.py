@@ -1,9 +1,10 @@
 """The launch schedules agree bit for bit: the flow schedule of long fits of many
-voxels with the grid schedule, which runs every iteration."""
+voxels with the grid schedule (which runs every iteration), and the random
+search with its draws side by side with one thread per voxel."""
 import pytest
 import torch
 
-from pycompute_gb300 import Expr, SecondOrderLevenbergMarquardt, pipeline, synth
+from pycompute_gb300 import Expr, SecondOrderLevenbergMarquardt, SecondOrderRandomSearch, pipeline, synth
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -40,4 +41,20 @@ def test_flow_equals_grid(workload, iters, kw):
         s.run(iters, block=block, **kw)
         torch.cuda.synchronize()
         got.append(_state(s))
+    _same(*got)
+
+
+@pytest.mark.parametrize("draws,lm_iters", [(1, 4), (3, 0), (7, 3), (130, 0)])
+def test_search_draws_side_by_side_equal_one_thread(draws, lm_iters):
+    w = synth.ivim()
+    n = 1 << 20
+    _, data = pipeline.synth_gpu(w, n, seed=4, device=DEV)
+    got = []
+    for m in (n, 701):  # many voxels: one thread each; few: the draws side by side
+        rs = SecondOrderRandomSearch(Expr(w.expr, w.pars, w.consts), w.M, torch.float32)
+        rs.setup(list(w.protocol), data[:, :m].contiguous(), list(w.lb), list(w.ub))
+        for seed in (11, 12):  # the second starts from the first one's best
+            rs.run(draws, lm_iters=lm_iters, seed=seed)
+        torch.cuda.synchronize()
+        got.append({"p": rs.best_pars_t[:, :701].contiguous(), "f": rs.best_f_t[:, :701].contiguous()})
     _same(*got)
