@@ -428,6 +428,20 @@ int pcgb_solve_helpers(int nparam, const float* A, const float* b, const float* 
 int pcgb_scalar_helpers(const float* a, const float* b, const double* x, float* root, float* quot, double* rcp,
                         float* prod, int32_t* ok, int64_t n, void* stream);
 
+/* First columns and column equality of up to three (rows, cols) device arrays
+ * (at most 256 rows each) in one launch and one copy back: values = the first
+ * columns as double, one array after the other, differs[k] = 1 where some column
+ * of array k differs from its first. scratch: PCGB_PROBE_HEADER + 8 * (sum of
+ * rows) bytes of device memory. Waits for the stream. */
+#define PCGB_PROBE_HEADER 16
+int pcgb_rows_probe(int count, const void* const* src, const int* rows, const int64_t* cols, int dtype, void* scratch,
+                    double* values, int* differs, void* stream);
+
+/* The state arrays of a fit that starts, in one launch: lam (n) = lam0, step
+ * (nparam, n) = 0, f (n) = 0, step_type (n) = 1, iters (n) = 0. */
+int pcgb_state_init(void* lam, void* step, void* f, int8_t* step_type, int32_t* iters, int64_t n, int nparam, int dtype,
+                    double lam0, void* stream);
+
 /* Constant initialisation: pars[k][v] = values[k]; a NaN entry means "the
  * voxel's largest sample" (the reference notebooks' S0 start). */
 int pcgb_init_constant(const float* data, int64_t n, int m, int nparam, const double* values, float* pars,

@@ -91,6 +91,9 @@ SIGNATURES = {
                                    c_void_p, c_void_p, c_i64, c_void_p]),
     "pcgb_scalar_helpers": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_i64, c_void_p]),
+    "pcgb_rows_probe": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "pcgb_state_init": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_i64, c_int, c_int, c_double,
+                                c_void_p]),
     "pcgb_copy_rows_async": (c_int, [c_void_p, c_i64, c_void_p, c_i64, c_i64, c_i64, c_int, c_void_p]),
     "pcgb_init_constant": (c_int, [c_void_p, c_i64, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "pcgb_bpolyfit": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_int, c_int, c_int, c_int, c_void_p,
@@ -171,7 +174,7 @@ def check(fn_name: str, rc: int):
         elif fn_name.startswith("pcgb_multi_run_noalloc"):
             err = L.pcgb_noalloc_last_error
         elif fn_name.startswith(("pcgb_init_constant", "pcgb_fp64_helpers", "pcgb_solve_helpers", "pcgb_scalar_helpers",
-                              "pcgb_copy_rows", "pcgb_fallback", "pcgb_bpolyfit", "pcgb_ivim")):
+                              "pcgb_rows_probe", "pcgb_state_init", "pcgb_copy_rows", "pcgb_fallback", "pcgb_bpolyfit", "pcgb_ivim")):
             err = L.pcgb_pipeline_last_error
         else:
             err = L.pcgb_last_error

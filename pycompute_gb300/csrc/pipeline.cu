@@ -8,6 +8,7 @@
 
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <string>
 
 #include "lm_params.h"
@@ -59,6 +60,58 @@ __global__ void scalar_helpers_kernel(const float* a, const float* b, const doub
   root[i] = pcgb::sqrt_fast(b[i]);
   quot[i] = pcgb::div_fast(a[i], b[i], pcgb::rcp_fast(b[i]));
   ok[i] = int(pcgb::rcp64_int(x[i], rcp[i])) | int(pcgb::scale_narrow(x[i], a[i], prod[i])) << 1;
+}
+
+// Rows of up to three (rows, cols) arrays given to a setup: their first column as
+// double, and per array whether any other column differs from it (NaN differs
+// from itself, as in a comparison of the arrays). Reading is all it does; one
+// launch and one copy back replace three of each.
+constexpr int kProbeArrays = 3;
+struct ProbeArgs {
+  const void* src[kProbeArrays];
+  int rows[kProbeArrays];
+  long long cols[kProbeArrays];
+  int count, is_double;
+  int* differs;    // [kProbeArrays], zeroed by the host
+  double* values;  // the first columns, one array after the other
+};
+template <typename T>
+__device__ void probe_rows(const ProbeArgs& a) {
+  const long long T_ = (long long)gridDim.x * blockDim.x, t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  int at = 0;
+  for (int k = 0; k < a.count; ++k) {
+    const T* s = static_cast<const T*>(a.src[k]);
+    bool differs = false;
+    for (int r = 0; r < a.rows[k]; ++r) {
+      const T* row = s + (long long)r * a.cols[k];
+      const T first = row[0];
+      if (t == 0) a.values[at + r] = double(first);
+      for (long long c = a.cols[k] > 1 ? t : a.cols[k]; c < a.cols[k]; c += T_) differs = differs || !(row[c] == first);
+    }
+    if (differs) a.differs[k] = 1;
+    at += a.rows[k];
+  }
+}
+__global__ void __launch_bounds__(256) probe_rows_kernel(const ProbeArgs a) {
+  if (a.is_double)
+    probe_rows<double>(a);
+  else
+    probe_rows<float>(a);
+}
+
+// The state of a fit that starts: damping, step codes, step, cost, iteration
+// counts, in one launch (five fills before).
+template <typename T>
+__global__ void __launch_bounds__(256) state_init_kernel(T* lam, T* step, T* f, signed char* step_type, int* iters,
+                                                         long long n, int nparam, double lam0) {
+  const long long T_ = (long long)gridDim.x * blockDim.x;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += T_) {
+    lam[v] = T(lam0);
+    f[v] = T(0);
+    step_type[v] = 1;
+    iters[v] = 0;
+    for (int k = 0; k < nparam; ++k) step[k * n + v] = T(0);
+  }
 }
 
 thread_local std::string g_err;
@@ -348,6 +401,63 @@ int pcgb_scalar_helpers(const float* a, const float* b, const double* x, float* 
   if (blocks > 0x7fffffffLL) return fail(PCGB_ERANGE, "scalar_helpers: n too large");
   scalar_helpers_kernel<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b, x, root, quot, rcp,
                                                                                          prod, ok, n);
+  return cuda_rc();
+}
+
+int pcgb_rows_probe(int count, const void* const* src, const int* rows, const int64_t* cols, int dtype, void* scratch,
+                    double* values, int* differs, void* stream) {
+  if (count < 1 || count > kProbeArrays || !src || !rows || !cols || !scratch || !values || !differs ||
+      (dtype != PCGB_DTYPE_F32 && dtype != PCGB_DTYPE_F64))
+    return fail(PCGB_EINVAL, "bad rows_probe arguments");
+  ProbeArgs a{};
+  int total = 0;
+  long long most = 1;
+  for (int k = 0; k < count; ++k) {
+    if (rows[k] < 0 || cols[k] < 1 || rows[k] > PCGB_MAX_PROTOCOL || (rows[k] > 0 && !src[k]))
+      return fail(PCGB_EINVAL, "rows_probe: 0..256 rows of at least one column");
+    a.src[k] = src[k];
+    a.rows[k] = rows[k];
+    a.cols[k] = cols[k];
+    total += rows[k];
+    if (cols[k] > most) most = cols[k];
+  }
+  a.count = count;
+  a.is_double = dtype == PCGB_DTYPE_F64;
+  a.differs = static_cast<int*>(scratch);
+  a.values = reinterpret_cast<double*>(static_cast<unsigned char*>(scratch) + PCGB_PROBE_HEADER);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemsetAsync(scratch, 0, PCGB_PROBE_HEADER, st);
+  if (e == cudaSuccess) {
+    const long long blocks = (most + 255) / 256;
+    probe_rows_kernel<<<unsigned(blocks < 1024 ? blocks : 1024), 256, 0, st>>>(a);
+    e = cudaGetLastError();
+  }
+  unsigned char host[PCGB_PROBE_HEADER + kProbeArrays * PCGB_MAX_PROTOCOL * sizeof(double)];
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(host, scratch, PCGB_PROBE_HEADER + size_t(total) * sizeof(double), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return fail(PCGB_ECUDA, cudaGetErrorString(e));
+  std::memcpy(differs, host, size_t(count) * sizeof(int));
+  std::memcpy(values, host + PCGB_PROBE_HEADER, size_t(total) * sizeof(double));
+  return PCGB_OK;
+}
+
+int pcgb_state_init(void* lam, void* step, void* f, int8_t* step_type, int32_t* iters, int64_t n, int nparam, int dtype,
+                    double lam0, void* stream) {
+  if (n < 0 || nparam < 1 || nparam > PCGB_MAX_PARAMS || (dtype != PCGB_DTYPE_F32 && dtype != PCGB_DTYPE_F64) ||
+      (n > 0 && (!lam || !step || !f || !step_type || !iters)))
+    return fail(PCGB_EINVAL, "bad state_init arguments");
+  if (n == 0) return PCGB_OK;
+  const long long need = (n + 255) / 256;
+  const unsigned blocks = unsigned(need < 4096 ? need : 4096);
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  signed char* codes = reinterpret_cast<signed char*>(step_type);
+  if (dtype == PCGB_DTYPE_F64)
+    state_init_kernel<<<blocks, 256, 0, st>>>(static_cast<double*>(lam), static_cast<double*>(step),
+                                              static_cast<double*>(f), codes, iters, n, nparam, lam0);
+  else
+    state_init_kernel<<<blocks, 256, 0, st>>>(static_cast<float*>(lam), static_cast<float*>(step),
+                                              static_cast<float*>(f), codes, iters, n, nparam, lam0);
   return cuda_rc();
 }
 

@@ -144,36 +144,77 @@ def _model_from(model_expr, f_gradf, legacy) -> tuple[str, str, int, int, str, O
     raise RuntimeError("One and only one of model_expr or f_gradf must be non None")
 
 
-def _shared_rows(t, rows: int, n: int, name: str, detect: bool):
-    """Classify a protocol/bounds argument: (device tensor or None, stride, host values).
-
-    A host sequence (list, tuple, numpy array, CPU tensor) of ``rows`` values
-    is a shared protocol and costs no device access; a (rows, 1) / (rows,)
-    CUDA tensor is shared too (read back once); a (rows, N) CUDA tensor is per
-    voxel unless ``detect`` finds all its columns equal.
-    """
+def _classify_rows(t, rows: int, n: int, name: str):
+    """One protocol/bounds argument: (values, None) for shared host values,
+    else (None, the (rows, cols) device tensor), cols 1 (shared) or n."""
     if not isinstance(t, torch.Tensor) and not hasattr(t, "__dlpack__"):
         vals = [float(x) for x in (t.reshape(-1) if hasattr(t, "reshape") else t)]
+    else:
+        t = _as_tensor(t, name)
+        vals = None if t.is_cuda else t.reshape(-1).double().tolist()
+    if vals is not None:
         if len(vals) != rows:
             raise RuntimeError(f"{name} must have {rows} values, got {len(vals)}")
-        return None, 0, vals
-    t = _as_tensor(t, name)
-    if not t.is_cuda:
-        vals = t.reshape(-1).double().tolist()
-        if len(vals) != rows:
-            raise RuntimeError(f"{name} must have {rows} values, got {len(vals)}")
-        return None, 0, vals
+        return vals, None
     if t.dim() == 1:
         t = t.reshape(rows, 1)
     if t.dim() != 2 or t.shape[0] != rows:
         raise RuntimeError(f"{name} must have {rows} rows, got shape {tuple(t.shape)}")
-    if t.shape[1] == 1 and n != 1:
-        return t, 0, t[:, 0].double().cpu().tolist()
-    if t.shape[1] != n:
+    if t.shape[1] != n and t.shape[1] != 1:
         raise RuntimeError(f"{name} must have 1 or {n} columns, got {t.shape[1]}")
-    if detect and n > 0 and bool((t == t[:, :1]).all()):
-        return t, 0, t[:, 0].double().cpu().tolist()
-    return t, n, None
+    return None, t
+
+
+def _shared_many(args, n: int, detect: bool):
+    """Classify protocol/bounds arguments [(t, rows, name), ...], at most three:
+    per argument (device tensor or None, stride, host values).
+
+    A host sequence (list, tuple, numpy array, CPU tensor) of ``rows`` values
+    is a shared protocol and costs no device access; a (rows, 1) / (rows,)
+    CUDA tensor is shared too (read back once); a (rows, N) CUDA tensor is per
+    voxel unless ``detect`` finds all its columns equal. All device arguments
+    are read back and compared by one launch and one copy (pcgb_rows_probe).
+    """
+    out = []
+    look = []  # (position, tensor) of the device arguments to read
+    for i, (t, rows, name) in enumerate(args):
+        vals, dev = _classify_rows(t, rows, n, name)
+        if dev is None:
+            out.append((None, 0, vals))
+        elif (dev.shape[1] == 1 and n != 1) or (detect and n > 0):
+            out.append((dev, 0, []))
+            if rows > 0:
+                look.append((i, dev))
+        else:
+            out.append((dev, n, None))
+    while look:
+        # the kernel reads float and double; anything else as double
+        read = [(i, t, (t if t.dtype in _TORCH_DTYPES else t.double()).contiguous()) for i, t in look]
+        dt, dv = read[0][2].dtype, read[0][2].device
+        read = [x for x in read if x[2].dtype == dt and x[2].device == dv]
+        look = [x for x in look if x[0] not in [y[0] for y in read]]
+        k, total = len(read), sum(t.shape[0] for _, _, t in read)
+        scratch = torch.empty(16 + 8 * total, dtype=torch.uint8, device=dv)
+        values, differs = (ctypes.c_double * total)(), (ctypes.c_int * k)()
+        with torch.cuda.device(dv):
+            rc = _lib.lib().pcgb_rows_probe(
+                k, (ctypes.c_void_p * k)(*[t.data_ptr() for _, _, t in read]),
+                (ctypes.c_int * k)(*[t.shape[0] for _, _, t in read]),
+                (ctypes.c_int64 * k)(*[t.shape[1] for _, _, t in read]), _TORCH_DTYPES[dt], _ptr(scratch), values,
+                differs, ctypes.c_void_p(_stream_ptr()))
+        _lib.check("pcgb_rows_probe", rc)
+        at = 0
+        for j, (i, t, r) in enumerate(read):
+            vals = values[at:at + r.shape[0]]
+            at += r.shape[0]
+            # one column equals itself unless it holds a NaN
+            out[i] = (t, n, None) if differs[j] or (n == 1 and any(v != v for v in vals)) else (t, 0, vals)
+    return out
+
+
+def _shared_rows(t, rows: int, n: int, name: str, detect: bool):
+    """_shared_many for one argument."""
+    return _shared_many([(t, rows, name)], n, detect)[0]
 
 
 def _parse_ctor(args, kwargs, names):
@@ -286,10 +327,10 @@ class SecondOrderLevenbergMarquardt:
         self.Nprobs = N
         self.pars_t = pars_t
         self.data_t = data_t
-        self.consts_t, self._cstride, self._protocol = _shared_rows(consts_t, C * M, N, "consts_t",
-                                                                      self.detect_shared)
-        self.lower_bound_t, bs_l, lbv = _shared_rows(lower_bound_t, P, N, "lower_bound_t", self.detect_shared)
-        self.upper_bound_t, bs_u, ubv = _shared_rows(upper_bound_t, P, N, "upper_bound_t", self.detect_shared)
+        ((self.consts_t, self._cstride, self._protocol), (self.lower_bound_t, bs_l, lbv),
+         (self.upper_bound_t, bs_u, ubv)) = _shared_many(
+            [(consts_t, C * M, "consts_t"), (lower_bound_t, P, "lower_bound_t"), (upper_bound_t, P, "upper_bound_t")],
+            N, self.detect_shared)
         if bs_l != bs_u:
             dev = pars_t.device
 
@@ -307,11 +348,14 @@ class SecondOrderLevenbergMarquardt:
         self.first_f = torch.empty((1, N), dtype=self.dtype, device=dev)
         self.last_f = torch.empty((1, N), dtype=self.dtype, device=dev)
         if init_state:
-            self.lam_t = torch.full((1, N), 5.0, dtype=self.dtype, device=dev)
-            self.step_t = torch.zeros((P, N), dtype=self.dtype, device=dev)
-            self.f_t = torch.zeros((1, N), dtype=self.dtype, device=dev)
-            self.step_type_t = torch.ones((1, N), dtype=torch.int8, device=dev)
-            self.iters_t = torch.zeros((1, N), dtype=torch.int32, device=dev)
+            self.lam_t, self.f_t = (torch.empty((1, N), dtype=self.dtype, device=dev) for _ in range(2))
+            self.step_t = torch.empty((P, N), dtype=self.dtype, device=dev)
+            self.step_type_t = torch.empty((1, N), dtype=torch.int8, device=dev)
+            self.iters_t = torch.empty((1, N), dtype=torch.int32, device=dev)
+            with torch.cuda.device(dev):
+                _lib.check("pcgb_state_init", _lib.lib().pcgb_state_init(
+                    _ptr(self.lam_t), _ptr(self.step_t), _ptr(self.f_t), _ptr(self.step_type_t), _ptr(self.iters_t),
+                    N, P, _TORCH_DTYPES[self.dtype], 5.0, ctypes.c_void_p(_stream_ptr())))
         else:
             self.lam_t = torch.empty((1, N), dtype=self.dtype, device=dev)
             self.f_t = torch.empty((1, N), dtype=self.dtype, device=dev)
