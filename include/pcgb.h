@@ -551,6 +551,39 @@ int pcgb_mlp_mse_grad(const float* y, const float* t, int64_t ldy, int64_t batch
 int pcgb_adam_step(float* master, float* m, float* v, float* grad, void* w_bf16, int64_t rows, int64_t ld,
                    int64_t rows_live, float lr, float b1, float b2, float eps, const float* corr, void* stream);
 
+/* Training steps of the 16 -> 128 -> 128 -> 128 -> nout network, two launches each:
+ * forward, mean-squared error, backward and weight gradients in one (tcgen05,
+ * 128 rows per CTA), Adam on all layers in the other. The arrays of layer l are
+ * (rows, in + 8) with rows 128, 128, 128, 8 and the bias in column `in`; w_bf16
+ * holds the masters rounded to bf16, grad is zero between steps. x_rows
+ * (n_batches * batch, 24) bf16 and targets (n_batches * batch, 8) as
+ * pcgb_mlp_prepare writes them; step s = first_step .. first_step + steps - 1
+ * takes batch s % n_batches and the Adam constants corr[3 s .. 3 s + 2] (bias
+ * corrections, learning-rate scale). batch is a multiple of 128. loss_sum (or
+ * NULL) is added to; status receives 1 if a bounded wait ran out (limit
+ * wait_limit, 0 = default; skip_block >= 0 makes one CTA never issue, for tests
+ * of that path). update 0 leaves the gradients and skips Adam. */
+typedef struct pcgb_mlp_train_net {
+  void* w_bf16[4];
+  float* master[4];
+  float* m[4];
+  float* v[4];
+  float* grad[4];
+  int nout;
+} pcgb_mlp_train_net;
+int pcgb_mlp_train_steps(const pcgb_mlp_train_net* net, const void* x_rows, const float* targets, int64_t n_batches,
+                         int64_t batch, int64_t first_step, int64_t steps, double lr, double b1, double b2, double eps,
+                         const float* corr, float* loss_sum, int* status, unsigned wait_limit, int64_t skip_block,
+                         int update, void* stream);
+/* Mean and standard deviation (population) of the transformed targets of a
+ * training set (kinds as in pcgb_mlp_prepare), in double, in one pass over
+ * signals (nin, n) and params (nout, n). scratch: PCGB_TARGET_STATS_DOUBLES
+ * doubles of device memory. Waits for the stream. */
+#define PCGB_TARGET_STATS_DOUBLES 4872
+int pcgb_mlp_train_target_stats(const float* signals, int nin, const float* params, int nout, const int* kinds,
+                                int64_t n, double* scratch, double* mean, double* stdv, void* stream);
+const char* pcgb_mlp_train_last_error(void);
+
 /* Training inputs x_rows (n x ldx) bf16 = signals / max per voxel (or
  * log(max(signals / max, 1e-6)) with log_in), column nin = 1; snorm[v] = that
  * maximum. With params/targets, also the normalised

@@ -131,6 +131,12 @@ SIGNATURES = {
                                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, ctypes.c_uint, c_i64,
                                        c_void_p]),
     "pcgb_mlp_tc_last_error": (c_char_p, []),
+    "pcgb_mlp_train_last_error": (c_char_p, []),
+    "pcgb_mlp_train_target_stats": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_i64, c_void_p, c_void_p,
+                                            c_void_p, c_void_p]),
+    "pcgb_mlp_train_steps": (c_int, [c_void_p, c_void_p, c_void_p, c_i64, c_i64, c_i64, c_i64, c_double, c_double,
+                                     c_double, c_double, c_void_p, c_void_p, c_void_p, ctypes.c_uint, c_i64, c_int,
+                                     c_void_p]),
 }
 
 
@@ -167,6 +173,8 @@ def check(fn_name: str, rc: int):
         L = lib()
         if fn_name.startswith("pcgb_gemm_bf16_tc"):
             err = L.pcgb_gemm_tc_last_error
+        elif fn_name.startswith("pcgb_mlp_train"):
+            err = L.pcgb_mlp_train_last_error
         elif fn_name.startswith("pcgb_mlp_forward_tc"):  # also pcgb_mlp_forward_tc_ex
             err = L.pcgb_mlp_tc_last_error
         elif fn_name.startswith(("pcgb_gemm", "pcgb_mlp", "pcgb_adam")):

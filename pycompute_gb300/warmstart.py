@@ -31,6 +31,12 @@ import torch
 from . import _lib
 
 HID = 128
+_STATS_DOUBLES = 4872  # PCGB_TARGET_STATS_DOUBLES
+
+
+class _TrainNet(ctypes.Structure):
+    _fields_ = [(k, ctypes.c_void_p * 4) for k in ("w_bf16", "master", "m", "v", "grad")] + [("nout", ctypes.c_int)]
+
 
 
 def _p(t):
@@ -144,6 +150,18 @@ class WarmStartMLP:
 
     def fit_normalisation(self, signals: torch.Tensor, params: torch.Tensor):
         """Mean / std of the transformed targets over a training set."""
+        if all(v.is_cuda and v.dtype == torch.float32 and v.dim() == 2 and v.is_contiguous() and v.shape[1] > 0
+               for v in (signals, params)) and signals.shape[1] == params.shape[1] and params.device == signals.device \
+                and signals.shape[0] > 0 and len(self.kinds) == self.nout <= params.shape[0]:
+            mean, std = (ctypes.c_double * self.nout)(), (ctypes.c_double * self.nout)()
+            with torch.cuda.device(signals.device):
+                scratch = torch.empty(_STATS_DOUBLES, dtype=torch.float64, device=signals.device)
+                _lib.check("pcgb_mlp_train_target_stats", _lib.lib().pcgb_mlp_train_target_stats(
+                    _p(signals), signals.shape[0], _p(params), self.nout, (ctypes.c_int * self.nout)(*self.kinds),
+                    signals.shape[1], _p(scratch), mean, std, _stream()))
+            for k in range(self.nout):
+                self.mean[k], self.std[k] = mean[k], max(std[k], 1e-6)
+            return
         smax = signals.max(dim=0).values.clamp_min(1e-20).double().cpu().numpy()
         p = params.double().cpu().numpy()
         for k, kind in enumerate(self.kinds):
@@ -231,9 +249,26 @@ class WarmStartMLP:
         self._backward(k_split)
         self._adam(lr)
 
+    def _fused_steps(self, x, t, n_batches: int, batch: int, first: int, steps: int, lr, corr, wait_limit: int = 0,
+                     skip_block: int = -1, update: bool = True):
+        """``steps`` training steps from step ``first`` of a run, two launches each (pcgb_mlp_train_steps)."""
+        if getattr(self, "_gemm_status", None) is None:
+            self._gemm_status = torch.zeros(1, dtype=torch.int32, device=self.device)
+        ptrs = lambda name: (ctypes.c_void_p * 4)(*[getattr(L, name).data_ptr() for L in self.layers])  # noqa: E731
+        net = _TrainNet(ptrs("wbf"), ptrs("master"), ptrs("m"), ptrs("v"), ptrs("grad"), self.nout)
+        rc = _lib.lib().pcgb_mlp_train_steps(ctypes.byref(net), _p(x), _p(t), n_batches, batch, first, steps, lr, 0.9,
+                                             0.999, 1e-8, _p(corr), _p(self.loss_sum), _p(self._gemm_status),
+                                             wait_limit, skip_block, int(update), _stream())
+        _lib.check("pcgb_mlp_train_steps", rc)
+
     def train(self, signals: torch.Tensor, params: torch.Tensor, epochs: int = 10, batch: int = 8192,
               lr: float = 2e-3, seed: int = 0, use_graph: bool = True, log_every: int = 0):
-        """Train on signals (nin, n) and label parameters (nout, n), both fp32 on the device."""
+        """Train on signals (nin, n) and label parameters (nout, n), both fp32 on the device.
+
+        With the tcgen05 GEMMs and batches of a multiple of 128 a step is two
+        launches (pcgb_mlp_train_steps) and ``use_graph`` has nothing to
+        capture; otherwise it is the sequence of GEMM, loss and Adam launches,
+        captured once and replayed."""
         with torch.cuda.device(self.device):
             self.fit_normalisation(signals, params)
             x, snorm, t = self._prepare(signals, params)
@@ -244,7 +279,11 @@ class WarmStartMLP:
             nb = n // batch
             if nb < 1:
                 raise ValueError("training set smaller than one batch")
-            self._alloc_batch(batch)
+            fused = self.gemm_impl == "tcgen05" and batch % 128 == 0
+            if fused:
+                self.loss_sum = torch.zeros(1, device=self.device)
+            else:
+                self._alloc_batch(batch)
             k_split = max(256, (batch // 32 + 31) // 32 * 32)
             b1, b2 = 0.9, 0.999
             graph = None
@@ -254,6 +293,17 @@ class WarmStartMLP:
             # the host queues steps ahead of the device)
             corr_tab = adam_step_constants(self.step, total, b1, b2).to(self.device)
             done = 0
+            if fused:
+                while done < total:
+                    k = min(log_every or total, total - done)
+                    self._fused_steps(x, t, nb, batch, done, k, lr, corr_tab)
+                    done += k
+                    self.step += k
+                    if log_every and done % log_every == 0:
+                        self.losses.append(float(self.loss_sum.item()) / log_every)
+                        self.loss_sum.zero_()
+                torch.cuda.synchronize()
+                return self
             for ep in range(epochs):
                 for b in range(nb):
                     self.bx.copy_(x[b * batch:(b + 1) * batch])
