@@ -303,8 +303,8 @@ int pcgb_model_eval(pcgb_fitter* fitter, const void* params, const void* consts,
 /* ---- mixed-model persistent batch (no reference counterpart) ----------------
  *
  * One program holds up to 8 models (each with its own protocol length); one
- * persistent launch fits every voxel of every model: warps claim chunks of
- * `chunk` voxels from a device work counter, so models with fast-converging
+ * persistent launch fits every voxel of every model: warps claim chunks of at
+ * most `chunk` voxels from a device work counter, so models with fast-converging
  * voxels hand their warps to the others. Protocols and bounds are shared per
  * model (host values in the job). The reference fits one model per program
  * and relaunches per iteration.
@@ -327,7 +327,7 @@ typedef struct {
 } pcgb_multi_job;
 
 /* Compile one program for n_models models (NVRTC, sm_103a, disk cache).
- * maxrreg: register cap (0 = compiler's choice); block: threads per block;
+ * maxrreg: registers per thread to build for (0 = the library's choice); block: threads per block;
  * lanes (may be NULL = all 1): per model, the warp lanes that share one
  * voxel (1 or 2; with 2 the two lanes split the voxel's samples and sum
  * their shares, so results match one lane's to float rounding). */

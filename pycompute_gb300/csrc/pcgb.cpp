@@ -159,9 +159,17 @@ constexpr int kLmFlowMinBlocks = 6;
 // flow: IVIM-10 x 100, 0.15 M voxels 1364, 1451, 0.3 M 2317, 2105, 1.2 M 8388,
 // 6090; x 64, 0.6 M 2784, 2820, 1.2 M 5417, 5129; x 50, 1.2 M 4264, 4731;
 // IVIM-21 x 64, 4.8 M 29966, 28126; T2*-16 x 64, 0.6 M 2572, 1311.
-constexpr int kFlowMinIters = 64;
+constexpr int kFlowMinIters = PCGB_FLOW_MIN_ITERS;
 constexpr int kFlowRestIters = 40;
 constexpr double kFlowMinWork = 128.0;
+// resident threads per SM that the mixed-model kernel is built for (VFA-8, T2*-16,
+// IVIM-10, biexp-T2-32, 262,147 voxels each x 100 iterations: 384 without a hint,
+// 512, 640, 768, 896 threads 17.0, 15.1, 14.7, 16.0, 16.2 ms)
+constexpr int kMultiThreads = 640;
+// claims of a warp that a mixed-model launch leaves at least: chunks are cut
+// down to that, so that the warps end together (the same: 64 voxels 16.0, 32 14.7
+// ms; 13.4 with the flow schedule for the three smaller models)
+constexpr int kMultiClaims = 8;
 constexpr int lm_min_blocks_of(int g) {
   return g == 1 ? kLmSearchMinBlocks : (g == 4 ? kLmWarmMinBlocks : (g == 3 ? kLmRefitMinBlocks : (g == 5 ? kLmFlowMinBlocks : kLmMinBlocks)));
 }
@@ -564,7 +572,7 @@ int kernel_of(pcgb_fitter* ft, int slot, cudaKernel_t* out) {
 static_assert(sizeof(PcgbMultiParams) <= 32000, "multi-model launch parameters exceed the 32 KB kernel parameter limit");
 
 std::string multi_source(int n, const char* const* srcs, const char* const* structs, const int* P, const int* C,
-                         const int* M, int dtype, int sdtype, int block, const int* lanes) {
+                         const int* M, int dtype, int sdtype, int block, int min_blocks, const int* lanes) {
   const char* ta = dtype == PCGB_DTYPE_F64 ? "double" : "float";
   const char* ts = sdtype == PCGB_DTYPE_F64 ? "double" : "float";
   std::ostringstream s;
@@ -581,18 +589,13 @@ std::string multi_source(int n, const char* const* srcs, const char* const* stru
     s << "static_assert(" << structs[k] << "::P == " << P[k] << " && " << structs[k] << "::C == " << C[k]
       << ", \"model shape\");\n";
   }
-  s << "struct PcgbDispatch {\n  static __device__ __forceinline__ void run(int k, const PcgbLmParams& a, long long base,"
-       " int chunk, int lane) {\n    switch (k) {\n";
-  // a model fitted with L lanes per voxel: lanes 2j, 2j + 1 (L = 2) share voxel j of each 16
-  for (int k = 0; k < n; ++k) {
-    const int L = lanes ? lanes[k] : 1;
-    s << "      case " << k << ":\n        for (int j = lane / " << L << "; j < chunk; j += " << 32 / L << ") {\n"
-      << "          const long long v = base + j;\n          if (v < a.N) pcgb::lm_fit_voxel<" << structs[k] << ", "
-      << M[k] << ", " << ta << ", " << ts << ", true, true, " << L << ">(a, v, pcgb::NoEpilogue{}, lane % " << L
-      << ");\n        }\n        break;\n";
-  }
-  s << "      default: break;\n    }\n  }\n};\n";
-  s << "extern \"C\" __global__ void __launch_bounds__(" << block
+  s << "struct PcgbDispatch {\n  static __device__ __forceinline__ unsigned run(int k, const PcgbMultiParams& q, int t,"
+       " unsigned c) {\n    switch (k) {\n";
+  for (int k = 0; k < n; ++k)
+    s << "      case " << k << ": return pcgb::multi_job<" << structs[k] << ", " << M[k] << ", " << ta << ", " << ts << ", "
+      << (lanes ? lanes[k] : 1) << ">(q, q.jobs[" << k << "], t, c);\n";
+  s << "      default: return 0xffffffffu;\n    }\n  }\n};\n";
+  s << "extern \"C\" __global__ void __launch_bounds__(" << block << ", " << min_blocks
     << ") pcgb_multi_lm(const PcgbMultiParams q) { pcgb::multi_grid<PcgbDispatch>(q); }\n";
   return s.str();
 }
@@ -690,10 +693,12 @@ int pcgb_multi_create(int n_models, const char* const* model_sources, const char
       return rc;
     if (lanes && lanes[k] != 1 && lanes[k] != 2) return fail(PCGB_EINVAL, "lanes per voxel must be 1 or 2");
   }
-  const std::string src =
-      multi_source(n_models, model_sources, model_structs, nparam, nconst, ndata, dtype, solve_dtype, block, lanes);
-  std::vector<std::string> extra;
-  if (maxrreg) extra.push_back("--maxrregcount=" + std::to_string(maxrreg));
+  // registers for kMultiThreads resident threads per SM, or as maxrreg says (as
+  // an occupancy hint: launch bounds override the compiler's register limit)
+  const int threads = maxrreg ? 65536 / maxrreg : (dtype == PCGB_DTYPE_F32 ? kMultiThreads : 0);
+  const std::string src = multi_source(n_models, model_sources, model_structs, nparam, nconst, ndata, dtype, solve_dtype,
+                                       block, threads / block > 1 ? threads / block : 1, lanes);
+  const std::vector<std::string> extra;
   std::vector<char> cubin;
   std::string log;
   if (int rc = cubin_for_source(src, extra, cache_dir, cubin, log)) return rc;
@@ -768,6 +773,13 @@ int pcgb_multi_run(pcgb_multi* m, const pcgb_multi_job* jobs, int n_jobs, const 
   int dev = -1;
   cudaGetDevice(&dev);
   if (dev != m->device) return fail(PCGB_EINVAL, "program was built on device %d but device %d is current", m->device, dev);
+  if (grid <= 0) grid = m->blocks_per_sm * m->sms;
+  {
+    double voxels = 0.0;
+    for (int k = 0; k < n_jobs; ++k) voxels += double(jobs[k].nprobs);
+    const double most = voxels / (double(grid) * (m->block / 32) * kMultiClaims);
+    if (most < chunk) chunk = most < 64.0 ? 32 : int(most) / 32 * 32;
+  }
   PcgbMultiParams q;
   std::memset(&q, 0, sizeof(q));
   q.counter = work_counter;
@@ -822,7 +834,6 @@ int pcgb_multi_run(pcgb_multi* m, const pcgb_multi_job* jobs, int n_jobs, const 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(work_counter, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
-  if (grid <= 0) grid = m->blocks_per_sm * m->sms;
   void* args[] = {&q};
   e = cudaLaunchKernel(reinterpret_cast<const void*>(m->kernel), dim3(grid), dim3(m->block), args, 0, s);
   if (e != cudaSuccess) return cuda_fail(e, "pcgb_multi_lm");
