@@ -32,8 +32,8 @@ def _solve(P, A, b, s, f, ftp, mu=0.25, eta=0.75):
     return x.cpu().numpy(), code.cpu().numpy()
 
 
-def _gmw64(A, b):
-    """The GMW81 solve (solver.py:23-95, 431-463): fp32 scaling, the rest in double, one system per column."""
+def _gmw64(A, b, out=np.float32):
+    """The GMW81 solve (solver.py:23-95, 431-463): scaling in A's type, the rest in double, one system per column."""
     P, n = b.shape
     rot = [P - 1] + list(range(P - 1))
     at = lambda i, j: A[max(i, j) * (max(i, j) + 1) // 2 + min(i, j)]  # noqa: E731
@@ -74,7 +74,7 @@ def _gmw64(A, b):
                 y[i] = y[i] - L[j][i] * y[j]
         x = [None] * P
         for i in range(P):
-            x[rot[i]] = (y[i] * (np.float32(1) / s[i]).astype(np.float64)).astype(np.float32)
+            x[rot[i]] = (y[i] * (A.dtype.type(1) / s[i]).astype(np.float64)).astype(out)
     return np.stack(x)
 
 
@@ -201,3 +201,24 @@ def test_integer_reciprocal_and_fp32_product_equal_the_fp64_ones():
     np.testing.assert_array_equal(prod.view(np.int32)[told], both.view(np.int32)[told])
     near = np.abs(np.log2(np.abs(np.where(x == 0, 1, x)))) < 25
     assert told[near & np.isfinite(x) & (x != 0)].mean() > 0.99 and not told[:8].any()
+
+
+@pytest.mark.parametrize("P", [2, 4, 6])
+@pytest.mark.parametrize("kind", ["definite", "indefinite", "zeros", "nan"])
+def test_double_solver_keeps_the_rules_of_its_maxima(P, kind):
+    """The all-double solve, whose maxima run on bit patterns, against the numpy rules (a NaN never wins)."""
+    from pycompute_gb300 import GMW81Solver
+
+    n = 1027
+    A, b = (v.astype(np.float64) for v in _systems(P, n, kind, np.random.default_rng(P + 50)))
+    x = torch.empty((P, n), dtype=torch.float64, device=DEV)
+    GMW81Solver(P, torch.float64).run(_t(A), _t(b), None, x)
+    got = x.cpu().numpy()
+    ref = _gmw64(A, b, np.float64)
+    fine = np.isfinite(ref)
+    np.testing.assert_array_equal(np.isfinite(got), fine)
+    d = np.sqrt(np.abs(np.stack([A[i * (i + 1) // 2 + i] for i in range(P)])))
+    with np.errstate(all="ignore"):
+        # rounding (2^-53) times the pivots' growth, as for the float solve above
+        bad = fine & (np.abs(got - ref) > 1e-9 * (np.abs(np.where(fine, ref, 0)) * d).max(0) / d + 1e-300)
+    assert bad.mean() < 1e-3, bad.mean()
