@@ -176,15 +176,20 @@ def _shared_many(args, n: int, detect: bool):
     are read back and compared by one launch and one copy (pcgb_rows_probe).
     """
     out = []
-    look = []  # (position, tensor) of the device arguments to read
-    for i, (t, rows, name) in enumerate(args):
-        vals, dev = _classify_rows(t, rows, n, name)
+    look = None  # (position, tensor) of the device arguments to read
+    for t, rows, name in args:
+        if type(t) is list:  # host values: the pipeline's setups pass nothing else
+            vals, dev = list(map(float, t)), None
+            if len(vals) != rows:
+                raise RuntimeError(f"{name} must have {rows} values, got {len(vals)}")
+        else:
+            vals, dev = _classify_rows(t, rows, n, name)
         if dev is None:
             out.append((None, 0, vals))
         elif (dev.shape[1] == 1 and n != 1) or (detect and n > 0):
             out.append((dev, 0, []))
             if rows > 0:
-                look.append((i, dev))
+                look = (look or []) + [(len(out) - 1, dev)]
         else:
             out.append((dev, n, None))
     while look:
