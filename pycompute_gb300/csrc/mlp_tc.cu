@@ -188,16 +188,22 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_infer_tc_kernel(const TcArgs p
   uint32_t phase = 0;
   bool lost = false;
 
+  // Tile t goes to CTA t mod gridDim.x, so that fewer tiles than 4 per SM spread
+  // over all SMs (four to a CTA, as before, and spread: 300 voxels 21.2, 17.0 us,
+  // 16,001 23.2, 17.0, 50,021 24.2, 21.1, 1 M 135.8, 131.7, 16.7 M 1873, 1837).
+  // The rest is latency: no pipe is above 56 % (ncu at 1 M: FMA-heavy 56, XU 46,
+  // issue 58, tensor 30 %), warps wait at the barriers of their tile's MMAs; two
+  // warpgroups per tile instead of one (1,024 threads) took 2.01 ms at 16.7 M.
   const long long ntiles = (p.n + 127) / 128;
-  const long long tstride = (long long)gridDim.x * NWG;
+  const long long tstride = (long long)gridDim.x * NWG, tile0 = (long long)g * gridDim.x + blockIdx.x;
   // signals of the next tile, loaded one tile ahead of their use
   float s_next[NIN];
   {
-    const long long v0 = ((long long)blockIdx.x * NWG + g) * 128 + r;
+    const long long v0 = tile0 * 128 + r;
 #pragma unroll
     for (int k = 0; k < NIN; ++k) s_next[k] = v0 < p.n ? p.signals[(long long)k * p.n + v0] : 0.f;
   }
-  for (long long tile = (long long)blockIdx.x * NWG + g; tile < ntiles && !lost; tile += tstride) {
+  for (long long tile = tile0; tile < ntiles && !lost; tile += tstride) {
     const long long v = tile * 128 + r;
     // ---- inputs: 16 samples of voxel v -> bf16 row r of x
     float s[NIN];
@@ -384,8 +390,7 @@ int pcgb_mlp_forward_tc_ex(const float* signals, int64_t n, int nin, int log_in,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms < 1) sms = 1;
   const long long tiles = (n + 127) / 128;
-  long long blocks = (tiles + NWG - 1) / NWG;
-  if (blocks > sms) blocks = sms;
+  const long long blocks = tiles < sms ? tiles : sms;
   mlp_infer_tc_kernel<<<unsigned(blocks), THREADS, smem, static_cast<cudaStream_t>(stream)>>>(a);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
