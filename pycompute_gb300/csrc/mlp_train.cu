@@ -22,7 +22,8 @@
 //     vector reductions.
 // What bounds it is the latency of that chain: 29 us for any batch up to 19,456
 // (issue 26 %, barriers a third of the stalls; two warpgroups instead of four
-// 33 us), 31 with the launches for 8,192 rows, 37 with Adam (105 before).
+// 33 us). With Adam a step of 8,192 rows takes 31.3 us (105 before; 37.0 with
+// ordinary launches in place of the dependent ones, see wait_for_previous).
 // Roundings (bf16 activations and gradients, fp32 sums) are those of the GEMM
 // path; only the order of the fp32 sums over rows differs.
 #include <cuda_bf16.h>
@@ -146,6 +147,15 @@ __device__ __forceinline__ void put16(bf16* tile, int r, int c, const uint32_t (
   *reinterpret_cast<uint4*>(p + 128) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
+// The launches of a run follow each other with programmatic dependent launch:
+// a kernel starts while the one before it still runs, does what needs nothing of
+// it, and waits here until that one has completed and its writes are visible.
+// The first launch of a call is an ordinary one, so whatever ran before it
+// (the batches' preparation) is complete for all of them; every kernel lets the
+// next one start only after its own wait, so two launches back is complete too.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __global__ void __launch_bounds__(THREADS, 1) mlp_train_step_kernel(const TrainArgs p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
@@ -155,15 +165,6 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_train_step_kernel(const TrainA
   const long long row0 = (long long)blockIdx.x * ROWS;
 
   stage_rows(S.x, p.x + row0 * LDX, ROWS, ROWS, NIN, LDX);
-  stage_rows(S.w1, p.w[0], HID, HID, NIN, LDX);
-  stage_rows(S.w2, p.w[1], HID, HID, HID, LDH);
-  stage_rows(S.w3, p.w[2], HID, HID, HID, LDH);
-  stage_rows(S.w4, p.w[3], 16, NOUT, HID, LDH);
-  for (int c = threadIdx.x; c < 3 * HID; c += THREADS) {
-    const int l = c / HID, n = c % HID;
-    S.bias[l][n] = l == 0 ? p.mw[0][n * LDX + NIN] : p.mw[l][n * LDH + HID];
-  }
-  if (threadIdx.x < NOUT) S.bias4[threadIdx.x] = p.mw[3][threadIdx.x * LDH + HID];
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.mbar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -174,6 +175,17 @@ __global__ void __launch_bounds__(THREADS, 1) mlp_train_step_kernel(const TrainA
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  wait_for_previous();
+  let_next_start();
+  stage_rows(S.w1, p.w[0], HID, HID, NIN, LDX);
+  stage_rows(S.w2, p.w[1], HID, HID, HID, LDH);
+  stage_rows(S.w3, p.w[2], HID, HID, HID, LDH);
+  stage_rows(S.w4, p.w[3], 16, NOUT, HID, LDH);
+  for (int c = threadIdx.x; c < 3 * HID; c += THREADS) {
+    const int l = c / HID, n = c % HID;
+    S.bias[l][n] = l == 0 ? p.mw[0][n * LDX + NIN] : p.mw[l][n * LDH + HID];
+  }
+  if (threadIdx.x < NOUT) S.bias4[threadIdx.x] = p.mw[3][threadIdx.x * LDH + HID];
   fence_async_smem();
   fence_before_sync();
   __syncthreads();
@@ -356,6 +368,8 @@ struct AdamArgs {
   const float* corr;     // bias corrections and learning-rate scale of this step
 };
 __global__ void __launch_bounds__(256) adam_all_kernel(const AdamArgs a) {
+  wait_for_previous();
+  let_next_start();
   int i = int(blockIdx.x) * 256 + int(threadIdx.x), l = 0;
   while (l < 4 && i >= a.size[l]) i -= a.size[l++];
   if (l == 4) return;
@@ -525,16 +539,29 @@ int pcgb_mlp_train_steps(const pcgb_mlp_train_net* net, const void* x_rows, cons
   a.b1 = float(b1);
   a.b2 = float(b2);
   a.eps = float(eps);
+  cudaLaunchAttribute pdl{};
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.stream = st;
+  cfg.attrs = &pdl;
   for (int64_t s = 0; s < steps; ++s) {
     const int64_t b = (first_step + s) % n_batches;
     p.x = static_cast<const bf16*>(x_rows) + b * batch * LDX;
     p.t = targets + b * batch * NOUT;
-    mlp_train_step_kernel<<<unsigned(batch / ROWS), THREADS, smem, st>>>(p);
-    if (update) {
+    cfg.gridDim = dim3(unsigned(batch / ROWS));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = size_t(smem);
+    cfg.numAttrs = s > 0 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, mlp_train_step_kernel, p);
+    if (e == cudaSuccess && update) {
       a.corr = corr + 3 * (first_step + s);
-      adam_all_kernel<<<unsigned((total + 255) / 256), 256, 0, st>>>(a);
+      cfg.gridDim = dim3(unsigned((total + 255) / 256));
+      cfg.blockDim = dim3(256);
+      cfg.dynamicSmemBytes = 0;
+      cfg.numAttrs = 1;
+      e = cudaLaunchKernelEx(&cfg, adam_all_kernel, a);
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess) return fail(PCGB_ECUDA, cudaGetErrorString(e));
   }
   return PCGB_OK;
