@@ -76,13 +76,14 @@ TOL = 1e-4
 METRIC = "IVIM voxel fits/s at 1e-4 rel err vs FP64: MLP-warm-start vs plain LM, 1 GB300"
 # network FLOPs per voxel: 2 * (16*128 + 128*128 + 128*128 + 128*4)
 NET_FLOP_PER_VOXEL = 2 * (16 * 128 + 2 * 128 * 128 + 128 * 4)
-# Binding-unit work per unit, from ncu opcode counts (sass__inst_executed per
-# opcode over one launch, divided by the units it processed): FP64-pipe
-# instructions (56 DFMA + 24 DMUL + 2 DADD) per IVIM-16 voxel-iteration of the
-# FP64-solve warm LM (4,194,304 warm-started voxels x 3 iterations) and MUFU
-# instructions per voxel of the tcgen05 network (1,048,576 IVIM-16 voxels;
-# 240 tanh for the 240 activations of the tanh columns, 16 log, 3 exp/rcp).
-FP64_OPS_PER_VOXEL_ITER = 82
+# Work per unit on the units that once bound the kernels, from ncu opcode counts
+# (sass__inst_executed per opcode over one launch, divided by the units it
+# processed): FP64-pipe instructions (warp instructions x 32; 22.2 DFMA and 10.3
+# DMUL by lanes that need them) per IVIM-16 voxel-iteration of the FP64-solve
+# warm LM (4,194,304 warm-started voxels x 3 iterations) and MUFU
+# instructions per voxel of the tcgen05 network (1,048,576 IVIM-16 voxels; 240
+# tanh for the 240 activations of the tanh columns, 16 log, 3 exp/rcp).
+FP64_OPS_PER_VOXEL_ITER = 45
 MUFU_PER_VOXEL_NET = 259
 # issue rates per SM per clock on sm_103a: FP64 at 1/64 of the 128 FP32 lanes,
 # MUFU 16 lanes
@@ -1151,7 +1152,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": lm_gbs, "peak": hbm, "unit": "GB/s", "frac": lm_gbs / hbm,
                          "traffic": traffic, "peak_source": peak_kind, "kernel": "pcgb_lmw (warm LM with the fallback check as its epilogue)",
                          "algorithmic_bytes_per_voxel": bpv, "kernel_ms": h["lm_ms"],
-                         "note": "per-voxel iterative solver: bound by the FP64 pipe (GMW81 solve + gain ratio), "
+                         "note": "per-voxel iterative solver: bound by instruction issue and the FP64 pipe, "
                                  "not by HBM; ncu summaries in profiles/"},
             "roofline_network": {"bound": "tensor", "achieved": net_tf, "peak": bf16_peak, "unit": "TFLOP/s",
                                  "frac": net_tf / bf16_peak, "kernel": "mlp_infer_tc_kernel (tcgen05)",
