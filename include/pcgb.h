@@ -112,6 +112,17 @@ int pcgb_lm_run(pcgb_fitter* fitter, const void* consts, int64_t consts_stride, 
                 void* stream);
 
 /*
+ * The launch schedule that pcgb_lm_run takes for nprobs voxels and iters
+ * iterations with shared protocol and bounds and block = 0 (per voxel the results
+ * are the same): PCGB_SCHEDULE_GRID, one thread per voxel, or PCGB_SCHEDULE_FLOW,
+ * a persistent grid whose lanes take a new voxel when theirs is done. Loads the
+ * kernel as pcgb_lm_run would. Negative: error.
+ */
+#define PCGB_SCHEDULE_GRID 0
+#define PCGB_SCHEDULE_FLOW 1
+int pcgb_lm_schedule(pcgb_fitter* fitter, int64_t nprobs, int iters, void* stream);
+
+/*
  * pcgb_lm_run restricted to the n_items voxels listed in vox_idx (int32
  * device array of distinct voxel indices < nprobs); all other voxels are left
  * untouched. Used to refit a compacted subset (the warm-start fallback) in

@@ -30,6 +30,7 @@ SIGNATURES = {
                                     c_size_t]),
     "pcgb_fitter_destroy": (c_int, [c_void_p]),
     "pcgb_fitter_log": (c_char_p, [c_void_p]),
+    "pcgb_lm_schedule": (c_int, [c_void_p, c_i64, c_int, c_void_p]),
     "pcgb_lm_run": (c_int, [c_void_p, c_void_p, c_i64, c_void_p, c_void_p, c_void_p, c_i64, c_double, c_double,
                             c_double, c_double, c_double, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                             c_void_p, c_void_p, c_i64, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,

@@ -7,6 +7,7 @@
 #define PCGB_MAX_PROTOCOL 256
 #define PCGB_MAX_MODELS 8
 #define PCGB_FLOW_MIN_ITERS 64  // iterations from which a fit may run the flow schedule
+#define PCGB_FLOW_MAX_PARAMS 4  // and the parameters up to which (the code of larger models outgrows the instruction cache)
 #define PCGB_MAX_SEARCH_BLOCK 128  // threads per block of the random search
 
 // PcgbLmParams.flags of an LM run

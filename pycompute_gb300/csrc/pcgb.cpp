@@ -83,6 +83,7 @@ struct pcgb_fitter {
   int device = -1;
   cudaLibrary_t lib[6] = {};  // one per kernel group, loaded on first use
   int lm_min_blocks[6] = {};  // occupancy hint the group's LM kernels were built with (0: none)
+  int flow = 0;               // the flow schedule's kernel: 0 not looked at yet, 1 loaded, -1 not for this model
   cudaKernel_t k[K_COUNT] = {};
   std::string source, structname, cache_dir;
   std::mutex mu;
@@ -484,11 +485,13 @@ int get_cubin(const char* model_source, const char* model_struct, int nparam, in
 }
 
 // Compile (or read from the cache) and load kernel group g of a fitter: first
-// with the LM kernels' occupancy hint, again without it if any of them spills
-// (local memory in use).
+// with the LM kernels' occupancy hint, again without it if any of them uses more
+// than kLmMaxSpillBytes of local memory (spills and the samples that the loops
+// index). The flow schedule's kernel has no second try: without its hint it does
+// not pay (see flow_kernel).
 int load_group(pcgb_fitter* ft, int g) {
   const int tries[2] = {lm_min_blocks_of(g), 0};
-  for (int t = 0; t < 2; ++t) {
+  for (int t = 0; t < (g == 5 ? 1 : 2); ++t) {
     if (t == 1 && tries[0] == 0) break;
     std::vector<char> cubin;
     std::string log;
@@ -531,21 +534,26 @@ int load_group(pcgb_fitter* ft, int g) {
   return fail(PCGB_ECOMPILE, "kernel group %d could not be loaded", g);
 }
 
-// Largest "N bytes spill stores" that ptxas reports for the register-capped
-// LM kernels in a compile log (0 if the log is empty, e.g. served from cache).
-size_t max_lm_spill_bytes(const std::string& log) {
+// The local memory per thread of the register-capped LM kernels in a compile log,
+// the largest: the stack with that of the functions they call, which load_group
+// judges by (it holds the samples that the loops index beside the spills), or the
+// spill stores where those are more (0 if the log is empty, e.g. served from
+// cache).
+size_t max_lm_local_bytes(const std::string& log) {
   size_t worst = 0;
   for (int slot = 0; slot < K_COUNT; ++slot) {
     if (!is_lm_slot(slot)) continue;
-    const std::string key = std::string("Function properties for ") + kKernelNames[slot] + "\n";
-    const size_t at = log.find(key);
+    const size_t at = log.find(std::string("Function properties for ") + kKernelNames[slot] + "\n");
     if (at == std::string::npos) continue;
-    const size_t sp = log.find("bytes spill stores", at);
-    if (sp == std::string::npos) continue;
-    size_t b = log.rfind(',', sp);
-    b = b == std::string::npos ? at : b + 1;
-    const size_t n = std::strtoull(log.c_str() + b, nullptr, 10);
-    if (n > worst) worst = n;
+    const size_t next = log.find("Function properties for ", at + 1);
+    const std::string part = log.substr(at, next == std::string::npos ? next : next - at);
+    for (const char* what : {" bytes stack frame", " bytes spill stores", " bytes cumulative stack size"}) {
+      const size_t end = part.find(what);
+      if (end == std::string::npos) continue;
+      const size_t before = part.find_last_not_of("0123456789", end - 1);
+      const size_t n = std::strtoull(part.c_str() + before + 1, nullptr, 10);
+      if (n > worst) worst = n;
+    }
   }
   return worst;
 }
@@ -567,6 +575,27 @@ int kernel_of(pcgb_fitter* ft, int slot, cudaKernel_t* out) {
   if (!ft->k[slot]) return fail(PCGB_EINVAL, "kernel %s missing from program", kKernelNames[slot]);
   *out = ft->k[slot];
   return PCGB_OK;
+}
+
+// The kernel of the flow schedule, or null for a model whose fits stay with the
+// grid: it pays only with its register cap, which no model of more than
+// PCGB_FLOW_MAX_PARAMS parameters keeps (a polynomial in 6 samples, 5 parameters:
+// 288 bytes of local memory; the bi-exponential in 32: 528), and of the others
+// those of few samples (IVIM in 10, 16, 21 samples: 160, 240, 272). A larger model
+// is therefore not compiled, and the answer, a kernel that fails to build
+// included, is kept: no call compiles again what an earlier one turned down. A
+// kernel that is not loaded yet is not loaded under stream capture.
+cudaKernel_t flow_kernel(pcgb_fitter* ft, void* stream) {
+  if (ft->P > PCGB_FLOW_MAX_PARAMS) return nullptr;
+  std::lock_guard<std::mutex> lock(ft->mu);
+  if (ft->flow == 0) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap) != cudaSuccess ||
+        cap != cudaStreamCaptureStatusNone)
+      return nullptr;
+    ft->flow = load_group(ft, 5) == PCGB_OK ? 1 : -1;
+  }
+  return ft->flow > 0 ? ft->k[K_LMF] : nullptr;
 }
 
 static_assert(sizeof(PcgbMultiParams) <= 32000, "multi-model launch parameters exceed the 32 KB kernel parameter limit");
@@ -624,7 +653,8 @@ int pcgb_fitter_compile(const char* model_source, const char* model_struct, int 
   if (int rc = validate_create(model_source, model_struct, nparam, nconst, ndata, dtype, solve_dtype)) return rc;
   std::string all;
   for (int g = 0; g < kGroups; ++g) {
-    if (g == 5 && (dtype != PCGB_DTYPE_F32 || solve_dtype != PCGB_DTYPE_F64)) continue;  // no kernel in it
+    // the flow schedule: one build, for the fitters that may run it
+    if (g == 5 && (dtype != PCGB_DTYPE_F32 || solve_dtype != PCGB_DTYPE_F64 || nparam > PCGB_FLOW_MAX_PARAMS)) continue;
     std::vector<char> cubin;
     std::string log;
     if (int rc = get_cubin(model_source, model_struct, nparam, nconst, ndata, dtype, solve_dtype, cache_dir, g,
@@ -632,7 +662,7 @@ int pcgb_fitter_compile(const char* model_source, const char* model_struct, int 
       return rc;
     // the register-capped LM kernels spill too much for this model: the
     // runtime will load the uncapped build, so compile (and cache) it too
-    if (max_lm_spill_bytes(log) > kLmMaxSpillBytes) {
+    if (g != 5 && max_lm_local_bytes(log) > kLmMaxSpillBytes) {
       all += log;
       log.clear();
       if (int rc = get_cubin(model_source, model_struct, nparam, nconst, ndata, dtype, solve_dtype, cache_dir, g, 0,
@@ -868,9 +898,7 @@ struct FallbackArgs {
   int8_t* which = nullptr;
 };
 
-// Whether a whole-volume fit runs the flow schedule (see kFlowMinIters), which
-// only pays where its kernel keeps the register cap. A kernel that is not loaded
-// yet is not loaded under stream capture.
+// Whether a whole-volume fit of n voxels runs the flow schedule (see kFlowMinIters).
 static bool flow_pays(pcgb_fitter* ft, int64_t n, int iters, void* stream) {
   if (ft->dtype != PCGB_DTYPE_F32 || ft->sdtype != PCGB_DTYPE_F64 || iters < kFlowMinIters) return false;
   int dev = 0, sms = 0;
@@ -878,11 +906,7 @@ static bool flow_pays(pcgb_fitter* ft, int64_t n, int iters, void* stream) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const double threads = double(kLmMaxThreads) * kLmFlowMinBlocks * (sms > 0 ? sms : 1);
   if (double(n) * (iters - kFlowRestIters) < kFlowMinWork * threads) return false;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap) != cudaSuccess) return false;
-  if (cap != cudaStreamCaptureStatusNone && !ft->k[K_LMF]) return false;
-  cudaKernel_t kern = nullptr;
-  return kernel_of(ft, K_LMF, &kern) == PCGB_OK && ft->lm_min_blocks[5] > 0;
+  return flow_kernel(ft, stream) != nullptr;
 }
 
 static int lm_run_impl(pcgb_fitter* ft, const void* consts, int64_t consts_stride, const void* data,
@@ -1009,6 +1033,14 @@ static int lm_run_impl(pcgb_fitter* ft, const void* consts, int64_t consts_strid
   if (block <= 0 && slot == K_LM_C1_B1 && !flags && flow_pays(ft, nprobs, iters, stream))
     return launch_resident(ft, K_LMF, prm, nprobs, block, stream);
   return launch(ft, slot, prm, nprobs, block, stream);
+}
+
+int pcgb_lm_schedule(pcgb_fitter* ft, int64_t nprobs, int iters, void* stream) {
+  g_err.clear();
+  if (!ft) return fail(PCGB_EINVAL, "fitter is NULL");
+  if (nprobs < 0 || iters < 0) return fail(PCGB_EINVAL, "nprobs and iters must be >= 0");
+  if (int rc = check_device(ft)) return rc;
+  return flow_pays(ft, nprobs, iters, stream) ? PCGB_SCHEDULE_FLOW : PCGB_SCHEDULE_GRID;
 }
 
 int pcgb_lm_run(pcgb_fitter* ft, const void* consts, int64_t consts_stride, const void* data,
