@@ -571,9 +571,11 @@ int pcgb_adam_step(float* master, float* m, float* v, float* grad, void* w_bf16,
  * pcgb_mlp_prepare writes them; step s = first_step .. first_step + steps - 1
  * takes batch s % n_batches and the Adam constants corr[3 s .. 3 s + 2] (bias
  * corrections, learning-rate scale). batch is a multiple of 128. loss_sum (or
- * NULL) is added to; status receives 1 if a bounded wait ran out (limit
- * wait_limit, 0 = default; skip_block >= 0 makes one CTA never issue, for tests
- * of that path). update 0 leaves the gradients and skips Adam. */
+ * NULL) is added to; status (or NULL) receives 1 if a bounded wait ran out
+ * (limit wait_limit, 0 = default; skip_block >= 0 makes one CTA never issue, for
+ * tests of that path), and while it is set the weights and moments stay as they
+ * are and the gradients are dropped. update 0 leaves the gradients and skips
+ * Adam. */
 typedef struct pcgb_mlp_train_net {
   void* w_bf16[4];
   float* master[4];

@@ -366,6 +366,7 @@ struct AdamArgs {
   int size[4], live[4];  // elements, and how many of them belong to live rows
   float lr, b1, b2, eps;
   const float* corr;     // bias corrections and learning-rate scale of this step
+  const int* status;     // set once a step's gradients are incomplete (see mlp_train_step_kernel), or null
 };
 __global__ void __launch_bounds__(256) adam_all_kernel(const AdamArgs a) {
   wait_for_previous();
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(256) adam_all_kernel(const AdamArgs a) {
   const float lr = a.lr * a.corr[2];
   const float gi = a.grad[l][i];
   a.grad[l][i] = 0.f;
-  if (i >= a.live[l]) return;
+  if (i >= a.live[l] || (a.status && *a.status)) return;  // nothing is learned from an incomplete gradient
   const float mi = a.b1 * a.m[l][i] + (1.f - a.b1) * gi;
   const float vi = a.b2 * a.v[l][i] + (1.f - a.b2) * gi * gi;
   a.m[l][i] = mi;
@@ -539,6 +540,7 @@ int pcgb_mlp_train_steps(const pcgb_mlp_train_net* net, const void* x_rows, cons
   a.b1 = float(b1);
   a.b2 = float(b2);
   a.eps = float(eps);
+  a.status = status;
   cudaLaunchAttribute pdl{};
   pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl.val.programmaticStreamSerializationAllowed = 1;

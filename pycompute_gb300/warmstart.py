@@ -268,8 +268,12 @@ class WarmStartMLP:
         With the tcgen05 GEMMs and batches of a multiple of 128 a step is two
         launches (pcgb_mlp_train_steps) and ``use_graph`` has nothing to
         capture; otherwise it is the sequence of GEMM, loss and Adam launches,
-        captured once and replayed."""
+        captured once and replayed. Raises RuntimeError if a tensor-core wait
+        ran out; with the two-launch steps the weights are then those before
+        the step that it happened in."""
         with torch.cuda.device(self.device):
+            if getattr(self, "_gemm_status", None) is not None:
+                self._gemm_status.zero_()
             self.fit_normalisation(signals, params)
             x, snorm, t = self._prepare(signals, params)
             n = x.shape[0]
@@ -302,8 +306,7 @@ class WarmStartMLP:
                     if log_every and done % log_every == 0:
                         self.losses.append(float(self.loss_sum.item()) / log_every)
                         self.loss_sum.zero_()
-                torch.cuda.synchronize()
-                return self
+                return self._trained()
             for ep in range(epochs):
                 for b in range(nb):
                     self.bx.copy_(x[b * batch:(b + 1) * batch])
@@ -328,7 +331,12 @@ class WarmStartMLP:
                     if log_every and done % log_every == 0:
                         self.losses.append(float(self.loss_sum.item()) / log_every)
                         self.loss_sum.zero_()
-            torch.cuda.synchronize()
+            return self._trained()
+
+    def _trained(self):
+        torch.cuda.synchronize()
+        if self.gemm_status():
+            raise RuntimeError("a wait for the tensor cores ran out during training: the network is not trained")
         return self
 
     # ---- inference ------------------------------------------------------------
