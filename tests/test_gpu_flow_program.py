@@ -92,3 +92,23 @@ def test_a_compiled_model_has_nothing_left_to_compile(tmp_path, monkeypatch, exp
     r.run(2, lm_iters=2, seed=1)
     torch.cuda.synchronize()
     assert set(os.listdir(tmp_path)) == programs
+
+
+def test_rest_in_long_fits_equals_grid():
+    """A damping that grows slowly: a voxel at rest has far more iterations left than its growth may span, until it has few
+    enough."""
+    w = synth.ivim()
+    iters = 1500
+    n = _least(iters) + 5
+    _, data = pipeline.synth_gpu(w, n, seed=9, device=DEV)
+    got = []
+    for block in (0, 128):
+        s = _fitter(w)
+        s.setup(pipeline.init_constant(data, w.init_values), list(w.protocol), data, list(w.lb), list(w.ub))
+        assert _schedule(s, n, iters) == "flow"
+        s.run(iters, dec=1.1, block=block)
+        got.append([getattr(s, k) for k in ("pars_t", "first_f", "last_f", "f_t", "lam_t", "step_type_t", "step_t",
+                                            "iters_t")])
+    for a, b in zip(*got):
+        a, b = (x.view(torch.int32) if x.dtype == torch.float32 else x for x in (a, b))
+        assert torch.equal(a, b)
