@@ -222,3 +222,17 @@ def test_double_solver_keeps_the_rules_of_its_maxima(P, kind):
         # rounding (2^-53) times the pivots' growth, as for the float solve above
         bad = fine & (np.abs(got - ref) > 1e-9 * (np.abs(np.where(fine, ref, 0)) * d).max(0) / d + 1e-300)
     assert bad.mean() < 1e-3, bad.mean()
+
+
+@pytest.mark.parametrize("P", [2, 3, 4, 5, 6])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_a_diagonal_that_is_not_finite_leaves_no_unknown(P, value):
+    """One such entry at every position, beside entries of every kind: no unknown is finite, as in the restatement."""
+    rng = np.random.default_rng(P + 90)
+    for kind in ("definite", "indefinite", "zeros"):
+        for i in range(P):
+            A, b = (v.copy() for v in _systems(P, 257, kind, rng))
+            A[i * (i + 1) // 2 + i] = value
+            x, _ = _solve(P, A, b, np.zeros_like(b), np.ones(257), np.ones(257))
+            assert not np.isfinite(_gmw64(A, b)).any()
+            assert not np.isfinite(x).any()
