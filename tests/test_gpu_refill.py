@@ -114,3 +114,15 @@ def test_refill_rejects_bad_schedule():
     solm = _setup(synth.ivim(), 64)
     with pytest.raises(ValueError):
         solm.run(5, schedule="bogus")
+
+
+@pytest.mark.parametrize("wl,M", [(synth.t2star, 8), (synth.t2star, 17), (synth.t2star, 31), (synth.t2star, 32),
+                                  (synth.ivim, 23), (synth.ivim, 24)])
+def test_refill_matches_grid_at_the_borders_of_whole_loops(wl, M):
+    """fp32 solve: sample loops whole in registers in one schedule, in both or in neither."""
+    import dataclasses
+
+    w = wl()
+    w = dataclasses.replace(w, protocol=[float(x) for x in np.linspace(w.protocol[0], w.protocol[-1], M)])
+    g, r = _pair(w, 5003, 40, solve=torch.float32)
+    _assert_same(_state(g), _state(r))
