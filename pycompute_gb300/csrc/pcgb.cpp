@@ -150,6 +150,12 @@ constexpr int kLmRefitMinBlocks = 6;
 // the random search (16,001 IVIM-21 voxels x 10 draws x 20 iterations: 4, 5 times
 // 964, 739 us; 6 spills more than kLmMaxSpillBytes)
 constexpr int kLmSearchMinBlocks = 5;
+// ... of a float32 fitter with the fp32 solve and three parameters. A refined draw
+// starts anywhere, its warps diverge, and resident warps are what hides that: T2*-16,
+// 60,000 voxels x 8 draws x 20 iterations at 5 and 8 times 966, 738 us, 1 M x 4 x 10
+// 2751, 2623. With the FP64 solve and two parameters the compiler's own choice, 62
+// registers with the loops rolled for it: VFA-8 1814, 875 and 6117, 3400 us.
+constexpr int kSearchFewMinBlocks = 8;
 // the flow schedule (4 M IVIM-10 voxels x 100 iterations: 5, 6, 7, 8 times 17.5,
 // 17.2, 17.5, 18.1 ms)
 constexpr int kLmFlowMinBlocks = 6;
@@ -194,6 +200,12 @@ std::string program_source(const char* model_source, const char* model_struct, i
   const std::string lmb = lm_min_blocks > 0 ? "__launch_bounds__(" + std::to_string(kLmMaxThreads) + ", " +
                                                   std::to_string(lm_min_blocks) + ")"
                                             : std::string(bounds);
+  // the random search (kLmSearchMinBlocks)
+  std::string rsb = lmb;
+  if (dtype == PCGB_DTYPE_F32 && lm_min_blocks > 0) {
+    if (P == 2 && sdtype == PCGB_DTYPE_F64) rsb = bounds;
+    if (P == 3 && sdtype == PCGB_DTYPE_F32) rsb = "__launch_bounds__(128, " + std::to_string(kSearchFewMinBlocks) + ")";
+  }
   const bool g0 = group == 0, g1 = group == 1, g2 = group == 2, g3 = group == 3, g4 = group == 4;
   if (group == 5 && dtype == PCGB_DTYPE_F32 && sdtype == PCGB_DTYPE_F64)
     s << "extern \"C\" __global__ void " << lmb << " pcgb_lmf(const PcgbLmParams a) { pcgb::lm_flow_grid<PcgbModel, " << M
@@ -236,7 +248,7 @@ std::string program_source(const char* model_source, const char* model_struct, i
       << (c ? "true" : "false") << ">(a); }\n";
   for (int c = 1; c >= 0 && g1; --c)
     for (int b = 1; b >= 0; --b)
-      s << "extern \"C\" __global__ void " << (c && b ? lmb : std::string("__launch_bounds__(128)")) << " pcgb_rs_c" << c << "_b" << b
+      s << "extern \"C\" __global__ void " << (c && b ? rsb : std::string("__launch_bounds__(128)")) << " pcgb_rs_c" << c << "_b" << b
         << "(const PcgbLmParams a) { pcgb::random_search_grid<PcgbModel, " << M << ", " << ta << ", " << ts << ", "
         << (c ? "true" : "false") << ", " << (b ? "true" : "false") << ">(a); }\n";
   for (int c = 1; c >= 0 && g2; --c) {

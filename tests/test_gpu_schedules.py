@@ -58,3 +58,30 @@ def test_search_draws_side_by_side_equal_one_thread(draws, lm_iters):
         torch.cuda.synchronize()
         got.append({"p": rs.best_pars_t[:, :701].contiguous(), "f": rs.best_f_t[:, :701].contiguous()})
     _same(*got)
+
+
+@pytest.mark.parametrize("workload,solve", [(synth.vfa_t1, torch.float64), (synth.vfa_t1, torch.float32),
+                                            (synth.t2star, torch.float64), (synth.t2star, torch.float32)])
+def test_search_of_few_parameters_equals_refined_starts(workload, solve):
+    """A draw refined by the search against the fitter started from that draw: with one draw, the parameters that the
+    search without refinement returns."""
+    w = workload()
+    n, iters = 4099, 20
+    _, data = pipeline.synth_gpu(w, n, seed=6, device=DEV)
+    got = []
+    for lm_iters in (0, iters):
+        rs = SecondOrderRandomSearch(Expr(w.expr, w.pars, w.consts), w.M, torch.float32, solve_dtype=solve)
+        rs.setup(list(w.protocol), data, list(w.lb), list(w.ub))
+        rs.run(1, lm_iters=lm_iters, seed=21)
+        got.append((rs.best_pars_t, rs.best_f_t.reshape(-1)))
+    p = got[0][0].clone()
+    s = SecondOrderLevenbergMarquardt(Expr(w.expr, w.pars, w.consts), None, w.M, torch.float32, solve_dtype=solve)
+    s.setup(p, list(w.protocol), data, list(w.lb), list(w.ub))
+    s.run(iters, block=128)
+    f = s.cost().reshape(-1)
+    torch.cuda.synchronize()
+    same = (got[1][0].view(torch.int32) == p.view(torch.int32)).all(0)
+    # the same arithmetic from the same start; a draw whose refinement stopped at the search's own start cost is kept
+    better = f < torch.finfo(torch.float32).max / 5
+    assert bool(same[better].all()), int((~same[better]).sum())
+    assert torch.equal(got[1][1][better].view(torch.int32), f[better].view(torch.int32))
