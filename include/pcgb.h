@@ -362,6 +362,12 @@ int pcgb_multi_run(pcgb_multi* program, const pcgb_multi_job* jobs, int n_jobs, 
                    double tol, double mu, double eta, double acc, double dec, int chunk, int grid,
                    uint32_t* work_counter, void* stream);
 
+/* The launch schedule (PCGB_SCHEDULE_GRID or PCGB_SCHEDULE_FLOW, see
+ * pcgb_lm_schedule) that the job of a program's model takes with nprobs voxels in
+ * a pcgb_multi_run of iters iterations and `grid` blocks (0 = the library's).
+ * Negative: error. */
+int pcgb_multi_schedule(const pcgb_multi* program, int model, int64_t nprobs, int iters, int grid);
+
 /*
  * pcgb_multi_run for callers that cannot allocate device memory. No reference
  * counterpart: the reference always allocates its buffers through CuPy.

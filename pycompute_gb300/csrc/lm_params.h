@@ -12,6 +12,7 @@
 
 // PcgbLmParams.flags of an LM run
 #define PCGB_LM_FRESH 1      // every voxel starts at lam = lam_start, step_type = 1; lam, f, step are not read
+#define PCGB_LM_FLOW 4       // a job of a mixed-model launch that runs the flow schedule
 #define PCGB_LM_PARS_ONLY 2  // only pars (and step_type, when given) are written back
 
 struct PcgbLmParams {

@@ -153,7 +153,7 @@ constexpr int kLmSearchMinBlocks = 5;
 // ... of a float32 fitter with the fp32 solve and three parameters. A refined draw
 // starts anywhere, its warps diverge, and resident warps are what hides that: T2*-16,
 // 60,000 voxels x 8 draws x 20 iterations at 5 and 8 times 966, 738 us, 1 M x 4 x 10
-// 2751, 2623. With the FP64 solve and two parameters the compiler's own choice, 62
+// 2751, 2623. With the FP64 solve and two parameters the compiler's own choice, 64
 // registers with the loops rolled for it: VFA-8 1814, 875 and 6117, 3400 us.
 constexpr int kSearchFewMinBlocks = 8;
 // the flow schedule (4 M IVIM-10 voxels x 100 iterations: 5, 6, 7, 8 times 17.5,
@@ -177,6 +177,14 @@ constexpr int kMultiThreads = 640;
 // down to that, so that the warps end together (the same: 64 voxels 16.0, 32 14.7
 // ms; 13.4 with the flow schedule for the three smaller models)
 constexpr int kMultiClaims = 8;
+// A job of a mixed-model launch runs the flow schedule from PCGB_FLOW_MIN_ITERS
+// iterations on and with this many voxels per thread of the launch: a lane needs
+// further voxels to turn to. us x 70 and x 100 iterations, grid and flow, VFA-8, T2*-16
+// and IVIM-10 of equal size in one launch of 97,280 threads: 0.03 voxels per thread
+// 470, 566 and 640, 680; 1.0 1700, 1957 and 2415, 2678; 2.1 3100, 2832 and 4365, 3487;
+// 5.1 7310, 5265 and 10286, 6106; about equal at 1.7 (x 64). (T2*-16 alone gains from
+// 0.9 on.)
+constexpr double kMultiFlowVoxels = 1.75;
 constexpr int lm_min_blocks_of(int g) {
   return g == 1 ? kLmSearchMinBlocks : (g == 4 ? kLmWarmMinBlocks : (g == 3 ? kLmRefitMinBlocks : (g == 5 ? kLmFlowMinBlocks : kLmMinBlocks)));
 }
@@ -644,8 +652,8 @@ std::string multi_source(int n, const char* const* srcs, const char* const* stru
 }  // namespace
 
 struct pcgb_multi {
-  int n = 0, dtype = 0, block = 128, device = -1;
-  int P[PCGB_MAX_MODELS] = {}, C[PCGB_MAX_MODELS] = {}, M[PCGB_MAX_MODELS] = {};
+  int n = 0, dtype = 0, sdtype = 0, block = 128, device = -1;
+  int P[PCGB_MAX_MODELS] = {}, C[PCGB_MAX_MODELS] = {}, M[PCGB_MAX_MODELS] = {}, lanes[PCGB_MAX_MODELS] = {};
   cudaLibrary_t lib = nullptr;
   cudaKernel_t kernel = nullptr;
   int blocks_per_sm = 0, sms = 0;
@@ -748,12 +756,14 @@ int pcgb_multi_create(int n_models, const char* const* model_sources, const char
   if (!m) return fail(PCGB_ENOMEM, "out of host memory");
   m->n = n_models;
   m->dtype = dtype;
+  m->sdtype = solve_dtype;
   m->block = block;
   m->log = log;
   for (int k = 0; k < n_models; ++k) {
     m->P[k] = nparam[k];
     m->C[k] = nconst[k];
     m->M[k] = ndata[k];
+    m->lanes[k] = lanes ? lanes[k] : 1;
   }
   cudaError_t e = cudaGetDevice(&m->device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
@@ -786,6 +796,25 @@ int pcgb_multi_destroy(pcgb_multi* m) {
 const char* pcgb_multi_log(const pcgb_multi* m) { return m ? m->log.c_str() : ""; }
 
 int pcgb_multi_grid(const pcgb_multi* m) { return m ? m->blocks_per_sm * m->sms : 0; }
+
+// Whether job k of a launch of `grid` blocks runs the flow schedule (see
+// kMultiFlowVoxels).
+static bool multi_flows(const pcgb_multi* m, int k, int64_t nprobs, int iters, int grid) {
+  if (m->dtype != PCGB_DTYPE_F32 || m->sdtype != PCGB_DTYPE_F64 || m->P[k] > PCGB_FLOW_MAX_PARAMS || m->lanes[k] != 1)
+    return false;
+  const int resident = m->blocks_per_sm * m->sms;
+  const double threads = double(grid < resident ? grid : resident) * m->block;
+  return iters >= PCGB_FLOW_MIN_ITERS && double(nprobs) >= kMultiFlowVoxels * threads;
+}
+
+int pcgb_multi_schedule(const pcgb_multi* m, int model, int64_t nprobs, int iters, int grid) {
+  g_err.clear();
+  if (!m) return fail(PCGB_EINVAL, "program is NULL");
+  if (model < 0 || model >= m->n || nprobs < 0 || iters < 0)
+    return fail(PCGB_EINVAL, "model outside the program, or nprobs or iters < 0");
+  if (grid <= 0) grid = m->blocks_per_sm * m->sms;
+  return multi_flows(m, model, nprobs, iters, grid) ? PCGB_SCHEDULE_FLOW : PCGB_SCHEDULE_GRID;
+}
 
 int pcgb_multi_run(pcgb_multi* m, const pcgb_multi_job* jobs, int n_jobs, const int* order, int iters, double tol,
                    double mu, double eta, double acc, double dec, int chunk, int grid, uint32_t* work_counter,
@@ -864,6 +893,7 @@ int pcgb_multi_run(pcgb_multi* m, const pcgb_multi_job* jobs, int n_jobs, const 
     a.N = j.nprobs;
     a.n_items = j.nprobs;
     a.iters = iters;
+    if (multi_flows(m, k, j.nprobs, iters, grid)) a.flags = PCGB_LM_FLOW;
     set_lm_constants(a, tol, mu, eta, acc, dec);
   }
   long long off = 0;
