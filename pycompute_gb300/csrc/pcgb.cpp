@@ -173,6 +173,13 @@ constexpr double kFlowMinWork = 128.0;
 // IVIM-10, biexp-T2-32, 262,147 voxels each x 100 iterations: 384 without a hint,
 // 512, 640, 768, 896 threads 17.0, 15.1, 14.7, 16.0, 16.2 ms)
 constexpr int kMultiThreads = 640;
+// ... and with a model of more than kMultiSmallParams parameters, whose spills at
+// 96 registers cost more than the threads gain (a sum of four exponentials, 8
+// parameters, FP64 solve: 848 bytes of stack at 640 threads, 688 at 512; 300,000
+// voxels x 20 iterations 4985, 4490 us, 4787 before the hint came; with 6
+// parameters, 384 bytes, 2035, 2012)
+constexpr int kMultiSmallParams = 6;
+constexpr int kMultiLargeThreads = 512;
 // claims of a warp that a mixed-model launch leaves at least: chunks are cut
 // down to that, so that the warps end together (the same: 64 voxels 16.0, 32 14.7
 // ms; 13.4 with the flow schedule for the three smaller models)
@@ -745,7 +752,10 @@ int pcgb_multi_create(int n_models, const char* const* model_sources, const char
   }
   // registers for kMultiThreads resident threads per SM, or as maxrreg says (as
   // an occupancy hint: launch bounds override the compiler's register limit)
-  const int threads = maxrreg ? 65536 / maxrreg : (dtype == PCGB_DTYPE_F32 ? kMultiThreads : 0);
+  int most = 0;
+  for (int k = 0; k < n_models; ++k) most = nparam[k] > most ? nparam[k] : most;
+  const int hint = most > kMultiSmallParams ? kMultiLargeThreads : kMultiThreads;
+  const int threads = maxrreg ? 65536 / maxrreg : (dtype == PCGB_DTYPE_F32 ? hint : 0);
   const std::string src = multi_source(n_models, model_sources, model_structs, nparam, nconst, ndata, dtype, solve_dtype,
                                        block, threads / block > 1 ? threads / block : 1, lanes);
   const std::vector<std::string> extra;

@@ -111,3 +111,29 @@ def test_two_lanes_per_voxel_match_one_lane():
         e2 = parity.compare_params(b[0], ref)["median_rel"]
         assert e2 <= 1.5 * e1 + 1e-7, (w.name, e1, e2)
         assert (b[2] > 0).all()
+
+
+@pytest.mark.parametrize("solve", [torch.float64, torch.float32])
+def test_eight_parameters_in_a_mixed_batch(solve):
+    """A model of the largest size (its program is built for fewer threads) beside a small one, against single fits."""
+    big = synth.Workload(
+        name="quad12", expr="S0*(f*exp(-b*D1)+g*exp(-b*D2)+h*exp(-b*D3)+(1-f-g-h)*exp(-b*D4))",
+        pars=["S0", "f", "g", "h", "D1", "D2", "D3", "D4"], consts=["b"], protocol=[80.0 * i for i in range(12)],
+        ranges=[(500, 1500), (.05, .2), (.1, .2), (.1, .2), (2e-2, 8e-2), (3e-3, 8e-3), (.5e-3, 1.5e-3), (1e-4, 3e-4)],
+        lb=[0, 0, 0, 0, 1e-3, 1e-4, 1e-8, 1e-8], ub=[20000, .999, .999, .999, .2, .02, .01, .01],
+        init_values=[float("nan"), .1, .1, .1, 3e-2, 5e-3, 1e-3, 2e-4])
+    ws = [big, synth.t2star()]
+    gens = [w.generate(777 + k, seed=70 + k) for k, w in enumerate(ws)]
+    fitter = MultiModelFitter([(Expr(w.expr, w.pars, w.consts), w.M) for w in ws], solve_dtype=solve)
+    jobs = _jobs(ws, gens)
+    fitter.fit(jobs, 1)
+    for w, (true, data, init, lb, ub, prot), j in zip(ws, gens, jobs):
+        s = SecondOrderLevenbergMarquardt(Expr(w.expr, w.pars, w.consts), None, w.M, torch.float32, solve_dtype=solve)
+        p = torch.from_numpy(init.copy()).to(DEV)
+        s.setup(p, list(prot), torch.from_numpy(data).to(DEV), list(lb), list(ub))
+        s.run(1)
+        torch.cuda.synchronize()
+        # one step in fp32 from the same start: the samples' sums may contract differently (2^-24 each), which the
+        # solve of an ill-conditioned system amplifies; most voxels agree to a few units
+        assert float((parity.rel_err(j.pars.cpu().numpy(), p.cpu().numpy()) <= 1e-4).mean()) > 0.98, w.name
+        assert parity.flags_agree(j.step_type.cpu().numpy(), s.step_type_t.cpu().numpy()) >= 0.98
