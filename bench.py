@@ -814,7 +814,7 @@ def mixed_batch_comparison(n_per_model=1 << 20, iters=100, seed=300):
         return jobs
 
     t0 = time.perf_counter()
-    tuned = autotune(models, lambda: make_jobs(0.125), iters=20)
+    tuned = autotune(models, lambda: make_jobs(0.125), iters=iters)
     tune_s = time.perf_counter() - t0
     fitter = MultiModelFitter(models, block=tuned["block"], maxrreg=tuned["maxrreg"], lanes=tuned.get("lanes"))
     fitter.chunk = tuned["chunk"]

@@ -362,6 +362,13 @@ int pcgb_multi_run(pcgb_multi* program, const pcgb_multi_job* jobs, int n_jobs, 
                    double tol, double mu, double eta, double acc, double dec, int chunk, int grid,
                    uint32_t* work_counter, void* stream);
 
+/* What the options of a mixed-model batch come to: the chunk that a run of
+ * `voxels` voxels over all jobs uses for `chunk`, and the resident blocks per SM
+ * that pcgb_multi_create builds for with `maxrreg` and `block` where the largest
+ * model has nparam parameters (equal blocks, equal program). Negative: error. */
+int pcgb_multi_chunk(const pcgb_multi* program, int64_t voxels, int chunk, int grid);
+int pcgb_multi_blocks(int nparam, int dtype, int maxrreg, int block);
+
 /* The launch schedule (PCGB_SCHEDULE_GRID or PCGB_SCHEDULE_FLOW, see
  * pcgb_lm_schedule) that the job of a program's model takes with nprobs voxels in
  * a pcgb_multi_run of iters iterations and `grid` blocks (0 = the library's).

@@ -80,6 +80,8 @@ SIGNATURES = {
     "pcgb_multi_destroy": (c_int, [c_void_p]),
     "pcgb_multi_log": (c_char_p, [c_void_p]),
     "pcgb_multi_grid": (c_int, [c_void_p]),
+    "pcgb_multi_chunk": (c_int, [c_void_p, c_i64, c_int, c_int]),
+    "pcgb_multi_blocks": (c_int, [c_int, c_int, c_int, c_int]),
     "pcgb_multi_schedule": (c_int, [c_void_p, c_int, c_i64, c_int, c_int]),
     "pcgb_multi_run": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_double, c_double, c_double, c_double,
                                c_double, c_int, c_int, c_void_p, c_void_p]),

@@ -667,6 +667,22 @@ struct pcgb_multi {
   std::string log;
 };
 
+// Resident blocks per SM that a mixed-model program of models of up to `nparam`
+// parameters is built for: registers for kMultiThreads resident threads, or as
+// maxrreg says (as an occupancy hint: launch bounds override the compiler's
+// register limit).
+static int multi_min_blocks(int nparam, int dtype, int maxrreg, int block) {
+  const int hint = nparam > kMultiSmallParams ? kMultiLargeThreads : kMultiThreads;
+  const int threads = maxrreg ? 65536 / maxrreg : (dtype == PCGB_DTYPE_F32 ? hint : 0);
+  return threads / block > 1 ? threads / block : 1;
+}
+// The chunk of a launch over `voxels` voxels: `chunk`, or what leaves every warp
+// kMultiClaims claims.
+static int multi_chunk(const pcgb_multi* m, double voxels, int chunk, int grid) {
+  const double most = voxels / (double(grid) * (m->block / 32) * kMultiClaims);
+  return most < chunk ? (most < 64.0 ? 32 : int(most) / 32 * 32) : chunk;
+}
+
 extern "C" {
 
 const char* pcgb_version(void) { return "pycompute-gb300 0.1 (sm_103a)"; }
@@ -750,14 +766,10 @@ int pcgb_multi_create(int n_models, const char* const* model_sources, const char
       return rc;
     if (lanes && lanes[k] != 1 && lanes[k] != 2) return fail(PCGB_EINVAL, "lanes per voxel must be 1 or 2");
   }
-  // registers for kMultiThreads resident threads per SM, or as maxrreg says (as
-  // an occupancy hint: launch bounds override the compiler's register limit)
   int most = 0;
   for (int k = 0; k < n_models; ++k) most = nparam[k] > most ? nparam[k] : most;
-  const int hint = most > kMultiSmallParams ? kMultiLargeThreads : kMultiThreads;
-  const int threads = maxrreg ? 65536 / maxrreg : (dtype == PCGB_DTYPE_F32 ? hint : 0);
   const std::string src = multi_source(n_models, model_sources, model_structs, nparam, nconst, ndata, dtype, solve_dtype,
-                                       block, threads / block > 1 ? threads / block : 1, lanes);
+                                       block, multi_min_blocks(most, dtype, maxrreg, block), lanes);
   const std::vector<std::string> extra;
   std::vector<char> cubin;
   std::string log;
@@ -792,6 +804,13 @@ int pcgb_multi_create(int n_models, const char* const* model_sources, const char
   return PCGB_OK;
 }
 
+int pcgb_multi_chunk(const pcgb_multi* m, int64_t voxels, int chunk, int grid) {
+  g_err.clear();
+  if (!m) return fail(PCGB_EINVAL, "program is NULL");
+  if (voxels < 0 || chunk < 32) return fail(PCGB_EINVAL, "voxels must be >= 0 and chunk >= 32");
+  return multi_chunk(m, double(voxels), chunk, grid > 0 ? grid : m->blocks_per_sm * m->sms);
+}
+
 int pcgb_multi_destroy(pcgb_multi* m) {
   if (!m) return PCGB_OK;
   int rc = PCGB_OK;
@@ -804,6 +823,13 @@ int pcgb_multi_destroy(pcgb_multi* m) {
 }
 
 const char* pcgb_multi_log(const pcgb_multi* m) { return m ? m->log.c_str() : ""; }
+
+int pcgb_multi_blocks(int nparam, int dtype, int maxrreg, int block) {
+  g_err.clear();
+  if (nparam < 1 || nparam > PCGB_MAX_PARAMS || (dtype != PCGB_DTYPE_F32 && dtype != PCGB_DTYPE_F64) || block < 32 || maxrreg < 0)
+    return fail(PCGB_EINVAL, "bad nparam, dtype, block or maxrreg");
+  return multi_min_blocks(nparam, dtype, maxrreg, block);
+}
 
 int pcgb_multi_grid(const pcgb_multi* m) { return m ? m->blocks_per_sm * m->sms : 0; }
 
@@ -855,12 +881,9 @@ int pcgb_multi_run(pcgb_multi* m, const pcgb_multi_job* jobs, int n_jobs, const 
   cudaGetDevice(&dev);
   if (dev != m->device) return fail(PCGB_EINVAL, "program was built on device %d but device %d is current", m->device, dev);
   if (grid <= 0) grid = m->blocks_per_sm * m->sms;
-  {
-    double voxels = 0.0;
-    for (int k = 0; k < n_jobs; ++k) voxels += double(jobs[k].nprobs);
-    const double most = voxels / (double(grid) * (m->block / 32) * kMultiClaims);
-    if (most < chunk) chunk = most < 64.0 ? 32 : int(most) / 32 * 32;
-  }
+  double voxels = 0.0;
+  for (int k = 0; k < n_jobs; ++k) voxels += double(jobs[k].nprobs);
+  chunk = multi_chunk(m, voxels, chunk, grid);
   PcgbMultiParams q;
   std::memset(&q, 0, sizeof(q));
   q.counter = work_counter;

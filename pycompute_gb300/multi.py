@@ -164,8 +164,18 @@ def _cache_path() -> str:
     return os.path.join(_build.BUILD, "autotune.json")
 
 
+def _library_id() -> str:
+    """Hash of the library: a choice timed with other kernels is not used again."""
+    with open(_build.LIB, "rb") as f:
+        return hashlib.sha1(f.read()).hexdigest()[:16]
+
+
+def _tune_key(gpu: str, fitter: MultiModelFitter, iters: int, lane_options) -> str:
+    return f"{gpu}|{_library_id()}|{fitter.key()}|{iters}|lanes{','.join(str(x) for x in lane_options)}"
+
+
 def autotune(models: list, make_jobs, iters: int, dtype=torch.float32, solve_dtype=None,
-             blocks=(64, 128, 256), maxrregs=(0, 128, 96), chunks=(32, 64, 128, 256), reps: int = 2,
+             blocks=(64, 128, 256), maxrregs=(0, 128, 255), chunks=(32, 64, 128, 256), reps: int = 2,
              use_cache: bool = True, lane_options=(1, 2)) -> dict:
     """Pick (block, maxrreg, chunk, order, lanes) for a model set.
 
@@ -173,11 +183,17 @@ def autotune(models: list, make_jobs, iters: int, dtype=torch.float32, solve_dty
     configuration is timed on it with CUDA events after one warm-up fit. The
     launch shape is searched with one lane per voxel; then, model by model,
     each other lanes-per-voxel option is tried on the best shape and kept if
-    the whole fit gets faster. The result is cached per GPU name and model set.
+    the whole fit gets faster. The result is cached per GPU name, library and
+    model set.
+
+    ``iters`` is the fits' own number of iterations, or one on the same side of
+    the flow schedule's limit of 64. Options that come to the same program or,
+    on this sample, to the same chunk are timed once; of such chunks the largest
+    stands, which on a larger batch leaves the cut to the launch.
     """
     probe = MultiModelFitter(models, dtype, solve_dtype)
     gpu = torch.cuda.get_device_name()
-    key = f"{gpu}|{probe.key()}|{iters}|lanes{','.join(str(x) for x in lane_options)}"
+    key = _tune_key(gpu, probe, iters, lane_options)
     path = _cache_path()
     cache = {}
     if use_cache and os.path.exists(path):
@@ -191,15 +207,27 @@ def autotune(models: list, make_jobs, iters: int, dtype=torch.float32, solve_dty
     inits = [j.pars.clone() for j in jobs]
     results = []
     t0 = time.perf_counter()
+    voxels = sum(j.N for j in jobs)
+    orders = [list(range(len(models)))]
+    if probe.heaviest_first() not in orders:
+        orders.append(probe.heaviest_first())
     for block in blocks:
+        built = set()
         for maxrreg in maxrregs:
+            program = _lib.lib().pcgb_multi_blocks(max(gm.P for gm, _ in probe.models), _TD[probe.dtype], maxrreg, block)
+            if program in built:
+                continue
+            built.add(program)
             fitter = MultiModelFitter(models, dtype, solve_dtype, block=block, maxrreg=maxrreg)
             try:
                 fitter.build()
             except _lib.PcgbError:
                 continue
-            for chunk in chunks:
-                for order in (list(range(len(models))), fitter.heaviest_first()):
+            cut = {}
+            for chunk in sorted(chunks):
+                cut[_lib.lib().pcgb_multi_chunk(fitter.build(), voxels, chunk, 0)] = chunk
+            for chunk in cut.values():
+                for order in orders:
                     times = []
                     for r in range(reps + 1):
                         for j, i0 in zip(jobs, inits):
