@@ -212,9 +212,11 @@ std::string program_source(const char* model_source, const char* model_struct, i
   s << "typedef " << model_struct << " PcgbModel;\n";
   s << "static_assert(PcgbModel::P == " << P << " && PcgbModel::C == " << C << ", \"model shape\");\n";
   const char* bounds = "__launch_bounds__(256)";
+  // (256, 1): left to itself the compiler takes 128 registers for the warm LM in
+  // double and spills 48 bytes; told that one block is enough it takes 140 and none
   const std::string lmb = lm_min_blocks > 0 ? "__launch_bounds__(" + std::to_string(kLmMaxThreads) + ", " +
                                                   std::to_string(lm_min_blocks) + ")"
-                                            : std::string(bounds);
+                                            : std::string(group == 4 ? "__launch_bounds__(256, 1)" : bounds);
   // the random search (kLmSearchMinBlocks)
   std::string rsb = lmb;
   if (dtype == PCGB_DTYPE_F32 && lm_min_blocks > 0) {
