@@ -78,9 +78,10 @@ METRIC = "IVIM voxel fits/s at 1e-4 rel err vs FP64: MLP-warm-start vs plain LM,
 NET_FLOP_PER_VOXEL = 2 * (16 * 128 + 2 * 128 * 128 + 128 * 4)
 # Work per unit on the units that once bound the kernels, from ncu opcode counts
 # (sass__inst_executed per opcode over one launch, divided by the units it
-# processed): FP64-pipe instructions (warp instructions x 32; 22.2 DFMA and 10.3
-# DMUL by lanes that need them) per IVIM-16 voxel-iteration of the FP64-solve
-# warm LM (4,194,304 warm-started voxels x 3 iterations) and MUFU
+# processed): FP64-pipe instructions per IVIM-16 voxel-iteration of the FP64-solve
+# warm LM (4,194,304 warm-started voxels x 3 iterations), as the pipe sees them: warp
+# instructions x 32, lanes that sit out a divergent path included (22.2 DFMA and 10.3
+# DMUL, 32.5 together, are by lanes that need them) and MUFU
 # instructions per voxel of the tcgen05 network (1,048,576 IVIM-16 voxels; 240
 # tanh for the 240 activations of the tanh columns, 16 log, 3 exp/rcp).
 FP64_OPS_PER_VOXEL_ITER = 45
@@ -814,7 +815,8 @@ def mixed_batch_comparison(n_per_model=1 << 20, iters=100, seed=300):
         return jobs
 
     t0 = time.perf_counter()
-    tuned = autotune(models, lambda: make_jobs(0.125), iters=iters)
+    # a quarter of the voxels: enough per thread to run the schedule that the whole batch runs
+    tuned = autotune(models, lambda: make_jobs(0.25), iters=iters)
     tune_s = time.perf_counter() - t0
     fitter = MultiModelFitter(models, block=tuned["block"], maxrreg=tuned["maxrreg"], lanes=tuned.get("lanes"))
     fitter.chunk = tuned["chunk"]

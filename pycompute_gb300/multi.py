@@ -187,9 +187,10 @@ def autotune(models: list, make_jobs, iters: int, dtype=torch.float32, solve_dty
     model set.
 
     ``iters`` is the fits' own number of iterations, or one on the same side of
-    the flow schedule's limit of 64. Options that come to the same program or,
-    on this sample, to the same chunk are timed once; of such chunks the largest
-    stands, which on a larger batch leaves the cut to the launch.
+    the flow schedule's limit of 64, and the sample is large enough to run the
+    schedule of the fits (1.75 voxels per thread and model). Options that come to the same program or,
+    on this sample, to the same chunk are timed once; of such chunks the smallest
+    stands, which on a larger batch spreads the end of the launch best.
     """
     probe = MultiModelFitter(models, dtype, solve_dtype)
     gpu = torch.cuda.get_device_name()
@@ -224,7 +225,7 @@ def autotune(models: list, make_jobs, iters: int, dtype=torch.float32, solve_dty
             except _lib.PcgbError:
                 continue
             cut = {}
-            for chunk in sorted(chunks):
+            for chunk in sorted(chunks, reverse=True):
                 cut[_lib.lib().pcgb_multi_chunk(fitter.build(), voxels, chunk, 0)] = chunk
             for chunk in cut.values():
                 for order in orders:

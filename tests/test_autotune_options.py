@@ -36,4 +36,4 @@ def test_no_option_is_timed_twice():
                           use_cache=False, lane_options=(1,))
     seen = [(t["block"], _lib.lib().pcgb_multi_blocks(3, 0, t["maxrreg"], t["block"]), tuple(t["order"])) for t in best["trials"]]
     assert len(seen) == len(set(seen)) == 4  # two blocks, two programs each; a few voxels cut every chunk to 32
-    assert best["chunk"] == 4096
+    assert best["chunk"] == 32
