@@ -137,7 +137,10 @@ bool is_fit_slot(int slot) {
 
 // their threads per block unless the caller says: single warps spread evenly over
 // the SMs and leave them one by one (65,536 IVIM-10 voxels x 10 iterations, all
-// FP64: 128, 64, 32 threads 2607, 2349, 2349 us; 50,000 x 50: 346, 342, 337)
+// FP64: 128, 64, 32 threads 2607, 2349, 2349 us; 50,000 x 50: 346, 342, 337). An SM
+// holds 32 blocks, which costs the smallest fp32 fitters, whose registers leave room
+// for 36 warps, up to 3 % (2 M VFA-8 voxels x 20, 128 and 32 threads: fp32 solve 2403,
+// 2469, FP64 solve 3203, 3250; T2*-16 2276, 2288 and 2616, 2613)
 constexpr int kFitBlock = 32;
 constexpr int kLmMinBlocks = 7;
 // the warm LM with the check as its epilogue (group 4; IVIM-16, 16.7 M voxels: 6,
@@ -164,8 +167,11 @@ constexpr int kLmFlowMinBlocks = 6;
 // first voxels come to rest: a pass there costs 20 to 35 % more than a grid
 // iteration (larger code, warps out of step) until voxels finish. us, grid and
 // flow: IVIM-10 x 100, 0.15 M voxels 1364, 1451, 0.3 M 2317, 2105, 1.2 M 8388,
-// 6090; x 64, 0.6 M 2784, 2820, 1.2 M 5417, 5129; x 50, 1.2 M 4264, 4731;
-// IVIM-21 x 64, 4.8 M 29966, 28126; T2*-16 x 64, 0.6 M 2572, 1311.
+// 6090; x 64, 0.6 M 2784, 2820, 1.2 M 5417, 5129; x 50, 1.2 M 4264, 4731; T2*-16 x 64,
+// 0.6 M 2572, 1311. A fit of 200 iterations and more flows as well: where voxels
+// converge it gains on (1 M T2*-16 x 400 26.4, 8.1 ms, VFA-8 21.8, 7.7), where most
+// only come to rest the damping overflows before the rest test applies, and the grid
+// is the faster one (1 M IVIM-10 x 200 18.9, 27.7 ms, x 400 38.2, 48.1).
 constexpr int kFlowMinIters = PCGB_FLOW_MIN_ITERS;
 constexpr int kFlowRestIters = 40;
 constexpr double kFlowMinWork = 128.0;
